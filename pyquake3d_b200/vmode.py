@@ -108,12 +108,15 @@ class MLPTrainer:
         loss = torch.zeros(1, dtype=torch.float32, device=self.dev)
         g = torch.Generator(device=self.dev)
         g.manual_seed(seed)
+        rows = B * max(1, (1 << 20) // B)
         for ep in range(epochs):
             perm = torch.randperm(N, device=self.dev, generator=g)
             loss.zero_()
             nb = 0
             for s in range(0, N - B + 1, B):
-                xb = data.index_select(0, perm[s:s + B]).contiguous()
+                if s % rows == 0:           # the next batches' samples in one gather
+                    x = data.index_select(0, perm[s:min(s + rows, N)])
+                xb = x[s % rows:s % rows + B]
                 self.step += 1
                 check(self.L.pq3d_mlp_train_step(ptr(self.P), ptr(self.M), ptr(self.V), ptr(xb), 6, ptr(xb[:, 5:]),
                                                  6, B, ptr(scratch), ptr(self.G), lr, 0.9, 0.999, 1e-8, self.step,
