@@ -118,6 +118,8 @@ __device__ void cta_max4(double *v, double *out)
     __syncthreads();
 }
 
+// TA: type of the matvec's slots.
+template <typename TA>
 __global__ void __launch_bounds__(ENS_THREADS) k_rk_ensemble(EnsArgs A)
 {
     __shared__ unsigned s_gen;
@@ -137,7 +139,10 @@ __global__ void __launch_bounds__(ENS_THREADS) k_rk_ensemble(EnsArgs A)
                 h = __ldcg(A.fstate + (int64_t)ENS_FSTATE * s);
             }
             // the H-matvec's row sums of the task's rows (one task is at most ENS_THREADS rows)
-            if (k == 0 && A.fuse_rowsum) rowsum_cta<ENS_THREADS>(A, A.task_row[t], A.task_row[t + 1]);
+            if (k == 0 && A.fuse_rowsum) {
+                const int r0 = A.task_row[t], r1 = A.task_row[t + 1];
+                rowsum_cta<ENS_THREADS, TA>(A, r0, r1, (r1 - r0 + 15) & ~15);
+            }
             double e4[4] = {0.0, 0.0, 0.0, 0.0};
             for (int64_t i = A.task_row[t] + threadIdx.x; i < A.task_row[t + 1]; i += ENS_THREADS) {
                 double e[4];
@@ -282,7 +287,10 @@ PQ3D_EXPORT int pq3d_ens_grid(int n_tasks)
     if (n_tasks <= 0) return -1;
     if (cudaGetDevice(&dev) != cudaSuccess) return -1;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_rk_ensemble, ENS_THREADS, 0) != cudaSuccess) return -1;
+    int per32 = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_rk_ensemble<double>, ENS_THREADS, 0) != cudaSuccess) return -1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per32, k_rk_ensemble<float>, ENS_THREADS, 0) != cudaSuccess) return -1;
+    per = per32 < per ? per32 : per;
     const int cap = sms * per;
     return n_tasks < cap ? n_tasks : cap;
 }
@@ -308,6 +316,6 @@ PQ3D_EXPORT int pq3d_ens_step(const void *args, int grid, cudaStream_t stream)
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    PQ3D_CHECK(cudaLaunchKernelEx(&cfg, k_rk_ensemble, A));
+    PQ3D_CHECK(cudaLaunchKernelEx(&cfg, A.slots_fp32 ? k_rk_ensemble<float> : k_rk_ensemble<double>, A));
     return PQ3D_OK;
 }

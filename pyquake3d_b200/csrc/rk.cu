@@ -26,8 +26,8 @@ struct RkArgs {
     const double *a, *b, *dc, *f0, *shear_loading, *normal_loading, *vplc, *cr0, *sr0;
     double *y;           // elastic load rates (n x 3): A1 x, A2 x, B x  (Pa/s)
     double *cand;        // 4n scratch
-    double *blk;         // 10 * gridDim + 16 scratch: per-CTA slip-rate maxima at [4G, 6G), the
-                         // grid maxima's three result slots (12 x u64) at 10G
+    double *blk;         // 10 * gridDim + 16 scratch: at 10G the grid maxima's three result slots
+                         // (12 x u64) and the slip-rate maxima (2 x u64); rows kernels: per-CTA maxima
     void *x;             // next deficit, interleaved (2n + padding), FP32 or FP64
     double *ctrl;        // control block (see pq3d.h)
     double *hist;        // per-step history, 6 doubles per step (may be null)
@@ -76,36 +76,44 @@ __device__ bool grid_max4(double *v, unsigned long long *slots3, unsigned *bar, 
     __shared__ int s_ok;
 #pragma unroll
     for (int q = 0; q < 4; ++q)
-#pragma unroll
+#pragma unroll 1
         for (int o = 16; o > 0; o >>= 1) v[q] = nanmax(v[q], __shfl_down_sync(0xffffffffu, v[q], o));
     if ((threadIdx.x & 31) == 0)
 #pragma unroll
         for (int q = 0; q < 4; ++q) wred[threadIdx.x >> 5][q] = v[q];
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
+        // lanes 0..3: one maximum each
         unsigned long long *r = slots3 + 4 * (attempt % 3);
-        double w[4] = {wred[0][0], wred[0][1], wred[0][2], wred[0][3]};
-        for (int k = 1; k < NT / 32; ++k)
-            for (int q = 0; q < 4; ++q) w[q] = nanmax(w[q], wred[k][q]);
-        for (int q = 0; q < 4; ++q) atomicMax(r + q, (unsigned long long)__double_as_longlong(w[q]));
-        const unsigned target = (unsigned)(attempt + 1) * gridDim.x;
-        int ok = 1;
-        if (atom_add_acq_rel_u32(bar, 1u) + 1u == target) {
-            unsigned long long *z = slots3 + 4 * ((attempt + 2) % 3);
-            for (int q = 0; q < 4; ++q) __stcg(z + q, 0ull);
-        } else {
-            long long it = 0;
-            while (ld_acquire_u32(bar) < target) {
-                if (++it > (1LL << 24)) {
-                    ctrl[4] = (double)PQ3D_ERR_TIMEOUT;
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(32);
-            }
+        const int q = threadIdx.x;
+        if (q < 4) {
+            double w = wred[0][q];
+            for (int k = 1; k < NT / 32; ++k) w = nanmax(w, wred[k][q]);
+            atomicMax(r + q, (unsigned long long)__double_as_longlong(w));
         }
-        for (int q = 0; q < 4; ++q) s_res[q] = __longlong_as_double((long long)__ldcg(r + q));
-        s_ok = ok;
+        __syncwarp();
+        if (q == 0) {
+            const unsigned target = (unsigned)(attempt + 1) * gridDim.x;
+            int ok = 1;
+            __threadfence();
+            if (atom_add_acq_rel_u32(bar, 1u) + 1u == target) {
+                unsigned long long *z = slots3 + 4 * ((attempt + 2) % 3);
+                for (int e = 0; e < 4; ++e) __stcg(z + e, 0ull);
+            } else {
+                long long it = 0;
+                while (ld_acquire_u32(bar) < target) {
+                    if (++it > (1LL << 24)) {
+                        ctrl[4] = (double)PQ3D_ERR_TIMEOUT;
+                        ok = 0;
+                        break;
+                    }
+                    __nanosleep(32);
+                }
+            }
+            s_ok = ok;
+        }
+        __syncwarp();
+        if (q < 4) s_res[q] = __longlong_as_double((long long)__ldcg(r + q));
     }
     __syncthreads();
 #pragma unroll
@@ -116,28 +124,36 @@ __device__ bool grid_max4(double *v, unsigned long long *slots3, unsigned *bar, 
 #ifndef PQ3D_RK_THREADS
 #define PQ3D_RK_THREADS 256
 #endif
-// Two 256-thread CTAs per SM (registers capped at 128, ~84 B spilled): at 60k
-// elements the co-resident grid then covers every element with one thread,
-// instead of two elements in half the threads at one CTA per SM (measured on
-// B200 at 60k: 49 us per step kernel instead of 61 us).
+// Two 256-thread CTAs per SM, R rows per CTA (rs_rows): at 60k elements one element per thread,
+// below that as few rows per CTA as fill the grid, so that all SMs share the latency-bound
+// element work and every thread the row sums.  B200, us per launch, against 256 rows per CTA:
+// 1,936 elements 47 -> 21, 9,000 33 -> 21, 20,480 24 -> 23, 60k 43 -> 38.  Cycles of a launch at
+// 20,480 (clock64 stamps): row sums 8,300, stages 14,900, grid maximum 7,900, accept 4,400,
+// end of step 5,300.
 #ifndef PQ3D_RK_MINB
 #define PQ3D_RK_MINB 2
 #endif
 constexpr int RK_THREADS = PQ3D_RK_THREADS;   // CTA size of the step kernel
 
+// TA: type of the matvec's slots (a kernel each, for half the code).
+template <typename TA>
 __global__ void __launch_bounds__(RK_THREADS, PQ3D_RK_MINB) k_rk_step(RkArgs A)
 {
     const int n = A.n;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const int64_t tid0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    // R rows per CTA, one per thread; the other threads take part in the row sums
+    const int R = pq3d::rs_rows(n, gridDim.x, RK_THREADS);
+    const int64_t stride = (int64_t)gridDim.x * R;
+    const int64_t tid0 = threadIdx.x < R ? (int64_t)blockIdx.x * R + threadIdx.x : n;
     if (A.fuse_rowsum) {
         // the H-matvec's row reduction (k_rowsum) done here: y[i] = sum of row i's slots
-        for (int64_t base = (int64_t)blockIdx.x * RK_THREADS; base < n; base += stride) rowsum_cta<RK_THREADS>(A, base, n);
+        for (int64_t base = (int64_t)blockIdx.x * R; base < n; base += stride)
+            rowsum_cta<RK_THREADS, TA>(A, base, n, R);
     }
     unsigned long long *slots3 = (unsigned long long *)(A.blk + 10 * (int64_t)gridDim.x);
     const bool forced = A.hforce != nullptr;
     StepCtl c{forced ? A.hforce[A.step_index] : (A.h_in > 0.0 ? A.h_in : A.ctrl[0]), 0.0, 0, 0, false};
     c.dtnext = c.h;
+    double E[4];
 
     while (true) {
         double m1 = 0.0, g1 = 0.0, g2 = 0.0, g3 = 0.0;  // max relative errors, NaN-propagating
@@ -150,11 +166,11 @@ __global__ void __launch_bounds__(RK_THREADS, PQ3D_RK_MINB) k_rk_step(RkArgs A)
             g3 = nanmax(g3, e[3]);
         }
         // grid-wide maxima of (m1, g1, g2, g3); identical in every CTA
-        double E[4] = {m1, g1, g2, g3};
+        E[0] = m1; E[1] = g1; E[2] = g2; E[3] = g3;
         if (!grid_max4<RK_THREADS>(E, slots3, A.bar, c.attempt, A.ctrl)) return;
-        if (controller(c, E, A.reltol, forced)) break;
+        if (controller_decide(c, E, A.reltol, forced)) break;
     }
-    const double h = c.h, dtnext = c.dtnext;
+    const double h = c.h;
     const bool accepted = c.accepted;
     const int nrjct = c.nrjct, attempt = c.attempt;
 
@@ -174,52 +190,35 @@ __global__ void __launch_bounds__(RK_THREADS, PQ3D_RK_MINB) k_rk_step(RkArgs A)
         mv2 = fmax(mv2, __shfl_down_sync(0xffffffffu, mv2, o));
     }
     __shared__ double vred[RK_THREADS / 32][2];
-    __shared__ int s_done;
     if ((threadIdx.x & 31) == 0) { vred[threadIdx.x >> 5][0] = mv1; vred[threadIdx.x >> 5][1] = mv2; }
     __syncthreads();
-    // the last CTA to finish the step reduces the slip-rate maxima and updates ctrl
+    // every CTA folds its slip-rate maxima (>= 0, never NaN) into two words; the last one to
+    // finish the step updates ctrl, read ahead of its arrival
     if (threadIdx.x == 0) {
         double w1 = vred[0][0], w2 = vred[0][1];
         for (int k = 1; k < RK_THREADS / 32; ++k) { w1 = fmax(w1, vred[k][0]); w2 = fmax(w2, vred[k][1]); }
-        A.blk[(int64_t)4 * gridDim.x + blockIdx.x] = w1;
-        A.blk[(int64_t)5 * gridDim.x + blockIdx.x] = w2;
+        const double c2 = A.ctrl[2], c4 = A.ctrl[4], c8 = A.ctrl[8], c9 = A.ctrl[9], c10 = A.ctrl[10];
+        atomicMax(slots3 + 12, (unsigned long long)__double_as_longlong(w1));
+        atomicMax(slots3 + 13, (unsigned long long)__double_as_longlong(w2));
         __threadfence();
-        s_done = atomicAdd(A.bar + 2, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!s_done) return;
-    __threadfence();
-    double w1 = 0, w2 = 0;
-    for (unsigned k = threadIdx.x; k < gridDim.x; k += RK_THREADS) {
-        w1 = fmax(w1, __ldcg(A.blk + (int64_t)4 * gridDim.x + k));
-        w2 = fmax(w2, __ldcg(A.blk + (int64_t)5 * gridDim.x + k));
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        w1 = fmax(w1, __shfl_down_sync(0xffffffffu, w1, o));
-        w2 = fmax(w2, __shfl_down_sync(0xffffffffu, w2, o));
-    }
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) { vred[threadIdx.x >> 5][0] = w1; vred[threadIdx.x >> 5][1] = w2; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        w1 = vred[0][0];
-        w2 = vred[0][1];
-        for (int k = 1; k < RK_THREADS / 32; ++k) { w1 = fmax(w1, vred[k][0]); w2 = fmax(w2, vred[k][1]); }
+        if (atomicAdd(A.bar + 2, 1u) != gridDim.x - 1) return;
+        __threadfence();
+        w1 = __longlong_as_double((long long)__ldcg(slots3 + 12));
+        w2 = __longlong_as_double((long long)__ldcg(slots3 + 13));
         A.bar[2] = 0u;
         A.bar[0] = 0u;
-        for (int q = 0; q < 12; ++q) slots3[q] = 0ull;
+        for (int q = 0; q < 14; ++q) slots3[q] = 0ull;
         if (accepted) {
-            const double t = A.ctrl[2] + h;
+            const double t = c2 + h, dtnext = controller_next(h, E, A.reltol);
             A.ctrl[2] = t;
             A.ctrl[0] = dtnext;   // next dttry
             A.ctrl[1] = h;        // accepted step
             A.ctrl[3] = nrjct;
             A.ctrl[5] = w1;
             A.ctrl[6] = w2;
-            A.ctrl[8] += 1.0;
-            A.ctrl[9] += nrjct;
-            A.ctrl[10] += attempt;
+            A.ctrl[8] = c8 + 1.0;
+            A.ctrl[9] = c9 + nrjct;
+            A.ctrl[10] = c10 + attempt;
             if (A.hist) {
                 double *hh = A.hist + 6 * (int64_t)A.step_index;
                 hh[0] = h; hh[1] = dtnext; hh[2] = t; hh[3] = w1; hh[4] = w2; hh[5] = nrjct;
@@ -227,7 +226,7 @@ __global__ void __launch_bounds__(RK_THREADS, PQ3D_RK_MINB) k_rk_step(RkArgs A)
         } else {
             A.ctrl[1] = h;
             A.ctrl[3] = nrjct;
-            if (A.ctrl[4] == 0.0) A.ctrl[4] = (double)PQ3D_ERR_DT;
+            if (c4 == 0.0) A.ctrl[4] = (double)PQ3D_ERR_DT;
         }
         if (A.ctrl_host) {
             // the host's copy, sequence number last (a step that ended early leaves it stale)
@@ -236,6 +235,12 @@ __global__ void __launch_bounds__(RK_THREADS, PQ3D_RK_MINB) k_rk_step(RkArgs A)
             A.ctrl_host[15] = (double)A.step_index + 1.0;
         }
     }
+}
+
+__device__ void rows_sum(const RkArgs &A, int64_t base, int64_t r1)
+{
+    if (A.slots_fp32) rowsum_cta<RK_THREADS, float>(A, base, r1, RK_THREADS);
+    else rowsum_cta<RK_THREADS, double>(A, base, r1, RK_THREADS);
 }
 
 // Row-range kernels of the row-partitioned (multi-GPU) step: the same element
@@ -283,9 +288,9 @@ __global__ void __launch_bounds__(RK_THREADS) k_rk_rows_attempt(RkArgs A, int r0
 {
     double e4[4] = {0.0, 0.0, 0.0, 0.0};
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    if (first && A.fuse_rowsum)   // the H-matvec's row sums, staged per CTA (same rows per thread as below)
+    if (first && A.fuse_rowsum)   // the H-matvec's row sums, staged per CTA (same rows per CTA as below)
         for (int64_t base = r0 + (int64_t)blockIdx.x * RK_THREADS; base < r1; base += stride)
-            rowsum_cta<RK_THREADS>(A, base, r1);
+            rows_sum(A, base, r1);
     for (int64_t i = r0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < r1; i += stride) {
         double e[4];
         dp54_element(A, i, h, e);
@@ -341,7 +346,7 @@ __global__ void __launch_bounds__(RK_THREADS) k_rk_rows_attempt_dev(RkArgs A, in
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     if (first && A.fuse_rowsum)
         for (int64_t base = r0 + (int64_t)blockIdx.x * RK_THREADS; base < r1; base += stride)
-            rowsum_cta<RK_THREADS>(A, base, r1);
+            rows_sum(A, base, r1);
     for (int64_t i = r0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < r1; i += stride) {
         double e[4];
         dp54_element(A, i, h, e);
@@ -419,13 +424,17 @@ PQ3D_EXPORT size_t pq3d_rk_args_bytes(void) { return sizeof(RkArgs); }
 // Largest co-resident grid for the step kernel on the current device.
 PQ3D_EXPORT int pq3d_rk_grid(int n)
 {
-    int dev = 0, sms = 0, per = 0;
+    int dev = 0, sms = 0, per = 0, per32 = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return -1;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_rk_step, RK_THREADS, 0) != cudaSuccess) return -1;
-    int need = (n + RK_THREADS - 1) / RK_THREADS;
-    int cap = sms * per;
-    return need < cap ? need : cap;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_rk_step<double>, RK_THREADS, 0) != cudaSuccess) return -1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per32, k_rk_step<float>, RK_THREADS, 0) != cudaSuccess) return -1;
+    per = per32 < per ? per32 : per;
+    const int64_t cap = (int64_t)sms * per;
+    if (n <= 0 || cap <= 0) return (int)(n < cap ? n : cap);
+    const int R = pq3d::rs_rows(n, cap, RK_THREADS);
+    const int64_t need = ((int64_t)n + R - 1) / R;
+    return (int)(need < cap ? need : cap);
 }
 
 static int rows_check(const RkArgs &A, int grid, int r0, int r1, const double *out)
@@ -518,7 +527,7 @@ PQ3D_EXPORT int pq3d_rk_step(const void *args, int grid, cudaStream_t stream)
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    PQ3D_CHECK(cudaLaunchKernelEx(&cfg, k_rk_step, A));
+    PQ3D_CHECK(cudaLaunchKernelEx(&cfg, A.slots_fp32 ? k_rk_step<float> : k_rk_step<double>, A));
     return PQ3D_OK;
 }
 
@@ -596,10 +605,10 @@ PQ3D_EXPORT int pq3d_rk_step_noalloc(const void *args, int grid, cudaStream_t st
     A.cand = s;
     A.blk = s + 4 * (size_t)PQ3D_NOALLOC_MAX_N;
     A.bar = (unsigned *)(s + 4 * (size_t)PQ3D_NOALLOC_MAX_N + 10 * (size_t)PQ3D_NOALLOC_MAX_GRID + 16);
-    // the barrier counters and the grid maxima's result slots (at blk + 10 * grid)
-    // must start at zero; the rest is written before it is read
+    // the barrier counters and the maxima's result slots (at blk + 10 * grid) must
+    // start at zero; the rest is written before it is read
     PQ3D_CHECK(cudaMemsetAsync(A.bar, 0, 4 * sizeof(unsigned), stream));
-    PQ3D_CHECK(cudaMemsetAsync(A.blk + 10 * (size_t)grid, 0, 12 * sizeof(unsigned long long), stream));
+    PQ3D_CHECK(cudaMemsetAsync(A.blk + 10 * (size_t)grid, 0, 14 * sizeof(unsigned long long), stream));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(RK_THREADS);
@@ -610,6 +619,6 @@ PQ3D_EXPORT int pq3d_rk_step_noalloc(const void *args, int grid, cudaStream_t st
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    PQ3D_CHECK(cudaLaunchKernelEx(&cfg, k_rk_step, A));
+    PQ3D_CHECK(cudaLaunchKernelEx(&cfg, A.slots_fp32 ? k_rk_step<float> : k_rk_step<double>, A));
     return PQ3D_OK;
 }

@@ -150,7 +150,12 @@ class Ensemble:
                        shear_loading=lambda s: s.shear_loading, normal_loading=lambda s: s.normal_loading,
                        vplc=lambda s: s.slipvC, cr0=lambda s: np.cos(s.rake0), sr0=lambda s: np.sin(s.rake0))
         self.t = {k: torch.tensor(np.ascontiguousarray(cat(g)), **f64) for k, g in getters.items()}
-        task_row, task_fault, fault_task = ensemble_tasks(self.struct.row0, self.L.pq3d_ens_task_rows())
+        # tasks as short as gives half the co-resident grid a task (in 16s), so that a small
+        # ensemble's row sums and element work spread over all SMs (12.6k elements: 28 us per
+        # step kernel with 96 rows, 33 with 256)
+        cap = max(1, self.L.pq3d_ens_grid(1 << 30) // 2)
+        rows = min(self.L.pq3d_ens_task_rows(), 16 * -(-n // (16 * cap)))
+        task_row, task_fault, fault_task = ensemble_tasks(self.struct.row0, rows)
         self.n_tasks = T = len(task_fault)
         self.task_row = torch.tensor(task_row, device=dev)
         self.task_fault = torch.tensor(task_fault, device=dev)
