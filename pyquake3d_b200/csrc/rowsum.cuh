@@ -95,7 +95,7 @@ __device__ __forceinline__ void rowsum_rows(const TA *__restrict__ slots, const 
         }
     }
     if (G == 1) {
-        if (r < rows) emit(r, a);
+        if (g == 0 && r < rows) emit(r, a);      // threads R.. NT have no row (R = 208: 48 of them)
         return;
     }
 #pragma unroll

@@ -77,3 +77,25 @@ def test_step_kernel_grids(prec, tmp_path):
     for g in got[1:]:
         for a, b in zip(g, got[0]):
             assert np.linalg.norm(np.asarray(a) - b) <= 1e-11 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("grid,rows", [(90, 16), (18, 80), (15, 96), (10, 144), (7, 208), (6, 240), (5, 256)])
+def test_step_kernel_row_sums(grid, rows, tmp_path):
+    """The step kernel's own row sums for CTAs of `rows` rows (threads left over in one and
+    several groups) equal the row reduction's, every time: 2 K 2^-53 of the largest product
+    for K slots a row."""
+    from pyquake3d_b200 import QDsim, meshgen, read_mshV2
+    from pyquake3d_b200.qdsim import DeviceStepper
+    msh, para = meshgen.make_case("thrust20k", str(tmp_path), n_target=1500, precision="fp64")
+    nodes, tris = read_mshV2(msh)
+    sim = QDsim(tris, nodes, para)
+    op = sim.tree_block.op()
+    st = DeviceStepper(sim, op, "fp64")
+    st.grid = grid
+    st.blk = torch.zeros(10 * st.grid + 16, dtype=torch.float64, device="cuda")
+    st.args["blk"] = st.blk.data_ptr()
+    assert st.n == 1428 and min(256, 16 * -(-st.n // (16 * grid))) == rows
+    for _ in range(40):
+        y = op.matvec(st.x, "fp64")
+        st.launch(0)
+        assert (st.y - y).abs().max() <= 1e-13 * y.abs().max()
