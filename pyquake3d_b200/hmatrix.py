@@ -198,16 +198,10 @@ def aca_start_indices(blocks, seed):
     (np.random.randint(n_rows) - 3, np.random.randint(n_cols) - 3 for the strike
     pass, then again for the dip pass, src/Hmatrix.py:660-661 and :888-889), with
     a seeded legacy RandomState and blocks taken in list order."""
-    rs = np.random.RandomState(seed)
-    out = []
-    for b in blocks:
-        if not b.aca:
-            continue
-        m, n = len(b.row.indices), len(b.col.indices)
-        s = (rs.randint(m) - 3, rs.randint(n) - 3)
-        d = (rs.randint(m) - 3, rs.randint(n) - 3)
-        out.append((s, d))
-    return out
+    sizes = [(len(b.row.indices), len(b.col.indices)) * 2 for b in blocks if b.aca]
+    # one draw over the array of bounds gives the numbers of a draw per bound
+    r = np.random.RandomState(seed).randint(np.array(sizes, dtype=np.int64).reshape(-1)) - 3
+    return [((a, b), (c, d)) for a, b, c, d in r.reshape(-1, 4).tolist()]
 
 
 # ----------------------------------------------------------------------------- packed layout (host)
@@ -230,17 +224,50 @@ def pack_x(x1, x2, n):
     return x
 
 
+def _expand(counts):
+    """For counts[i] consecutive items of each owner i: (owner, index within the owner)."""
+    counts = np.asarray(counts, dtype=np.int64)
+    owner = np.repeat(np.arange(len(counts)), counts)
+    return owner, np.arange(len(owner)) - (np.cumsum(counts) - counts)[owner]
+
+
+def _offsets(sizes):
+    """Exclusive running sum of sizes, and the total."""
+    t = np.cumsum(sizes, dtype=np.int64)
+    return t - sizes, int(t[-1]) if len(t) else 0
+
+
+def _fields(dtype, n, **cols):
+    """n records of `dtype` from columns (at least one zero record, for the uploads)."""
+    rec = np.zeros(max(n, 1), dtype=dtype)
+    for k, v in cols.items():
+        rec[k][:n] = v
+    return rec
+
+
+def _block_geometry(blocks):
+    """(m, n, first row, first column, lo, hi) of blocks in tree order; [lo, hi) are the
+    block-local rows the plan computes (all, unless a row partition clipped them)."""
+    g = np.array([(len(b.row.indices), len(b.col.indices), b.row.start, b.col.start) + getattr(b, "rows", (0, -1))
+                  for b in blocks], dtype=np.int64).reshape(-1, 6).T
+    return g[0], g[1], g[2], g[3], g[4], np.where(g[5] < 0, g[0], g[5])
+
+
 def dense_layout(dense_blocks):
     """DenseBlock records with FP64 / FP32 offsets, and the two array sizes.  Stored
     columns start at the column-group-aligned c0 - (c0 % CW)."""
+    m, n, r0, c0, _, _ = _block_geometry(dense_blocks)
+    off64, n64 = _offsets(_cdiv(n + c0 % 2, 2) * m * 12)
+    off32, n32 = _offsets(_cdiv(n + c0 % 4, 4) * m * 24)
     recs = np.zeros(len(dense_blocks), dtype=_lib.DENSE_BLOCK)
-    off64 = off32 = 0
-    for i, b in enumerate(dense_blocks):
-        m, n, c0 = len(b.row.indices), len(b.col.indices), b.col.start
-        recs[i] = (off64, off32, m, n, b.row.start, c0)
-        off64 += _cdiv(n + c0 % 2, 2) * m * 12
-        off32 += _cdiv(n + c0 % 4, 4) * m * 24
-    return recs, off64, off32
+    for k, v in dict(off64=off64, off32=off32, m=m, n=n, r0=r0, c0=c0).items():
+        recs[k] = v
+    return recs, n64, n32
+
+
+_PACK = np.dtype([("bi", "i8"), ("pass_", "i8"), ("u_off", "i8"), ("v_off", "i8"), ("K", "i8"), ("Q", "i8"), ("kS", "i8"),
+                  ("kD", "i8")])
+_PACK_M = np.dtype([("bi", "i8"), ("pass_", "i8")] + [(k, "i8", 3) for k in ("u_off", "v_off", "kS", "kD", "Q", "K", "sb")])
 
 
 def build_plan_arrays(struct, dense_recs, kS, kD, code, dense_chunk=64, v_chunk=256, u_rows=512):
@@ -254,78 +281,81 @@ def build_plan_arrays(struct, dense_recs, kS, kD, code, dense_chunk=64, v_chunk=
     cwd, cwl = _CW_DENSE[code], _CW_LR[code]
     n = struct.n
     dense_off = dense_recs["off64"] if code == 0 else dense_recs["off32"]
-    ditems, slot_rows, slot = _dense_items(dense_recs, cwd, dense_off, dense_chunk)
-    aca_blocks = [b for b in struct.blocks if b.aca]
-    u_off = v_off = tp = 0
-    vitems, utasks, pack = [], [], []
-    lr_entries = 0
-    kmax = 0
-    for bi, b in enumerate(aca_blocks):
-        m, nn = len(b.row.indices), len(b.col.indices)
-        lo, hi = getattr(b, "rows", (0, m))      # block-local rows this plan computes (all, unless clipped)
-        ks, kd = int(kS[bi]), int(kD[bi])
-        lr_entries += 3 * (ks + kd) * ((hi - lo) + nn)
-        if ks + kd == 0:
-            continue
-        K = _cdiv(ks + kd, cwl) * cwl
-        kmax = max(kmax, K)
-        Q = 3 * (ks + kd)
-        lead = b.col.start % cwl
-        ngv = _cdiv(nn + lead, cwl)
-        npad = ngv * cwl
-        nch = _cdiv(ngv, v_chunk)
-        for ch in range(nch):
-            g0 = ch * v_chunk
-            g1 = min(ngv, g0 + v_chunk)
-            for s_, (qa, qb) in enumerate(((0, 3 * ks), (3 * ks, Q))):
-                for q in range(qa, qb, 32):
-                    vitems.append((v_off, Q, q, min(32, qb - q), g0, g1, b.col.start - lead, s_, tp + ch * Q))
-        # row r of the block writes slot (slot - lo) + r, for r in [lo, hi)
-        for r0 in range(lo, hi, u_rows):
-            utasks.append((u_off, m, r0, min(hi, r0 + u_rows), K, ks, kd, Q, tp, nch, slot - lo))
-        slot_rows.append((slot, b.row.start + lo, hi - lo))
-        for p in (0, 1):
-            pack.append((bi, p, u_off, v_off, K, Q, ks, kd))
-        slot += hi - lo
-        tp += nch * Q
-        u_off += (K // cwl) * m * 3 * cwl
-        v_off += Q * npad
+    ditems, slot_rows, slot0 = _dense_items(dense_recs, cwd, dense_off, dense_chunk)
+    m, nn, row0, c0, lo, hi = _block_geometry([b for b in struct.blocks if b.aca])
+    ks, kd = np.asarray(kS, np.int64)[:len(m)], np.asarray(kD, np.int64)[:len(m)]
+    lr_entries = int((3 * (ks + kd) * ((hi - lo) + nn)).sum())
+    on = np.nonzero(ks + kd > 0)[0]                     # blocks with terms
+    m, nn, row0, c0, lo, hi, ks, kd = (a[on] for a in (m, nn, row0, c0, lo, hi, ks, kd))
+    K, Q, lead = _cdiv(ks + kd, cwl) * cwl, 3 * (ks + kd), c0 % cwl
+    ngv = _cdiv(nn + lead, cwl)
+    nch = _cdiv(ngv, v_chunk)
+    u_off, u_size = _offsets((K // cwl) * m * 3 * cwl)
+    v_off, v_size = _offsets(Q * ngv * cwl)
+    tp, n_tpart = _offsets(nch * Q)
+    slot, n_slots = _offsets(hi - lo)
+    slot, n_slots = slot + slot0, n_slots + slot0
+    # V items: per column chunk, the strike rows then the dip rows, 32 to an item
+    nS, nD = _cdiv(3 * ks, 32), _cdiv(3 * kd, 32)
+    b, i = _expand(nch * (nS + nD))
+    ch, i = i // (nS + nD)[b], i % (nS + nD)[b]
+    dip = i >= nS[b]
+    q = np.where(dip, 3 * ks[b] + 32 * (i - nS[b]), 32 * i)
+    nv = len(b)
+    vitems = _fields(_lib.V_ITEM, nv, off=v_off[b], Q=Q[b], q=q, nr=np.minimum(32, np.where(dip, Q[b], 3 * ks[b]) - q),
+                     g0=ch * v_chunk, g1=np.minimum(ngv[b], (ch + 1) * v_chunk), c0=(c0 - lead)[b], s=dip,
+                     tp=tp[b] + ch * Q[b])
+    # U tasks; row r of the block writes slot (slot - lo) + r, for r in [lo, hi)
+    b, i = _expand(_cdiv(hi - lo, u_rows))
+    r0 = lo[b] + i * u_rows
+    nu = len(b)
+    utasks = _fields(_lib.U_TASK, nu, off=u_off[b], m=m[b], r0=r0, r1=np.minimum(hi[b], r0 + u_rows), K=K[b], kS=ks[b],
+                     kD=kd[b], Q=Q[b], tp=tp[b], nch=nch[b], slot=(slot - lo)[b])
+    slot_rows = np.concatenate([slot_rows, np.stack([slot, row0 + lo, hi - lo], axis=1)])
+    pack = np.zeros(2 * len(on), dtype=_PACK)
+    for k, v in dict(bi=on, u_off=u_off, v_off=v_off, K=K, Q=Q, kS=ks, kD=kd).items():
+        pack[k] = np.repeat(v, 2)
+    pack["pass_"] = np.tile([0, 1], len(on))
     L = _leaf_lists(struct, slot_rows)
     esz_d = 8 if code == 0 else 4
     esz_l = {0: 8, 1: 4, 2: 2}[code]
     dense_entries = int(np.sum(dense_recs["m"].astype(np.int64) * dense_recs["n"])) if len(dense_recs) else 0
-    return dict(ditems=_rec(ditems, _lib.DENSE_ITEM), vitems=_rec(vitems, _lib.V_ITEM),
-                utasks=_rec(utasks, _lib.U_TASK),
-                n_ditems=len(ditems), n_vitems=len(vitems), n_utasks=len(utasks), n_slots=slot, n_tpart=tp, kmax=kmax,
-                u_size=u_off, v_size=v_off, pack=pack, alg_bytes=dense_entries * 6 * esz_d + lr_entries * esz_l +
+    nd = len(ditems)
+    return dict(ditems=_fields(_lib.DENSE_ITEM, 0) if nd == 0 else ditems, vitems=vitems, utasks=utasks,
+                n_ditems=nd, n_vitems=nv, n_utasks=nu, n_slots=n_slots, n_tpart=n_tpart,
+                kmax=int(K.max()) if len(K) else 0,
+                u_size=u_size, v_size=v_size, pack=pack, alg_bytes=dense_entries * 6 * esz_d + lr_entries * esz_l +
                 2 * n * esz_d + 3 * n * 8, **L)
 
 
 def _dense_items(dense_recs, cwd, dense_off, dense_chunk):
     """Dense work items (one warp: 32 rows x a chunk of column groups) and their slots:
     every (block, column chunk) owns m consecutive slots."""
-    ditems, slot_rows = [], []
-    slot = 0
-    for i in range(len(dense_recs)):
-        m, nn, r0, c0 = (int(dense_recs[k][i]) for k in ("m", "n", "r0", "c0"))
-        lead = c0 % cwd
-        ng = _cdiv(nn + lead, cwd)
-        for g0 in range(0, ng, dense_chunk):
-            g1 = min(ng, g0 + dense_chunk)
-            for r in range(0, m, 32):
-                ditems.append((int(dense_off[i]), m, r, g0, g1, c0 - lead, slot))
-            slot_rows.append((slot, r0, m))
-            slot += m
-    return ditems, slot_rows, slot
+    m, nn, r0, c0 = (dense_recs[k].astype(np.int64) for k in ("m", "n", "r0", "c0"))
+    lead = c0 % cwd
+    ng = _cdiv(nn + lead, cwd)
+    nch, nr = _cdiv(ng, dense_chunk), _cdiv(m, 32)
+    ob, ch = _expand(nch)                              # slot owners: (block, column chunk)
+    slot, n_slots = _offsets(m[ob])
+    o, i = _expand(nr[ob])
+    b = ob[o]
+    ditems = np.zeros(len(o), dtype=_lib.DENSE_ITEM)
+    for k, v in dict(off=np.asarray(dense_off)[b], m=m[b], r=32 * i, g0=ch[o] * dense_chunk,
+                     g1=np.minimum(ng[b], (ch[o] + 1) * dense_chunk), c0=(c0 - lead)[b], slot=slot[o]).items():
+        ditems[k] = v
+    return ditems, np.stack([slot, r0[ob], m[ob]], axis=1).reshape(-1, 3), n_slots
 
 
 def _leaf_lists(struct, slot_rows):
     """Per leaf cluster, the offsets (slot - first row) of every slot owner covering it."""
     n = struct.n
     nleaf = len(struct.leaves)
-    leaf_of_row = np.empty(n, dtype=np.int32)
-    for lf in struct.leaves:
-        leaf_of_row[lf.start:lf.start + len(lf.indices)] = lf.leaf_id
+    start = np.array([lf.start for lf in struct.leaves], dtype=np.int64)
+    leaf_id = np.array([lf.leaf_id for lf in struct.leaves], dtype=np.int32)
+    leaf_of_row = np.repeat(leaf_id, [len(lf.indices) for lf in struct.leaves])
+    if len(start) and (np.diff(start) < 0).any():      # leaves listed out of row order
+        order = np.argsort(start, kind="stable")
+        leaf_of_row = np.repeat(leaf_id[order], [len(struct.leaves[i].indices) for i in order])
     sr = np.array(slot_rows, dtype=np.int64).reshape(-1, 3)
     first = leaf_of_row[sr[:, 1]].astype(np.int64)
     last = leaf_of_row[sr[:, 1] + sr[:, 2] - 1].astype(np.int64)
@@ -334,9 +364,7 @@ def _leaf_lists(struct, slot_rows):
     rep_off = np.repeat(sr[:, 0] - sr[:, 1], cnt)
     order = np.argsort(rep_leaf, kind="stable")
     leaf_off = rep_off[order].astype(np.int32)
-    leaf_ptr = np.zeros(nleaf + 1, dtype=np.int64)
-    np.add.at(leaf_ptr, rep_leaf + 1, 1)
-    leaf_ptr = np.cumsum(leaf_ptr).astype(np.int32)
+    leaf_ptr = np.concatenate([[0], np.cumsum(np.bincount(rep_leaf, minlength=nleaf))]).astype(np.int32)
     return dict(leaf_of_row=leaf_of_row, leaf_ptr=leaf_ptr,
                 leaf_off=leaf_off if len(leaf_off) else np.zeros(1, np.int32), slot_rows=sr)
 
@@ -383,12 +411,45 @@ def classify_terms(wS, wD, tol):
     return cls[:len(wS)], cls[len(wS):]
 
 
+def classify_blocks(w, offs, tol):
+    """classify_terms over all blocks at once: w holds every term's weight in task order
+    (block by block, strike terms then dip), offs the tasks' offsets (two per block and
+    the total).  Returns the class of every term."""
+    K = offs[2::2] - offs[:-1:2]
+    blk = np.repeat(np.arange(len(K)), K)
+    first = (np.cumsum(K) - K)[blk]
+    w = w[:len(blk)]
+    req = np.where(2 * MIXED_EPS[1] * w > tol, 0, np.where(2 * MIXED_EPS[2] * w > tol, 1, 2))
+    n0 = np.bincount(blk[req == 0], minlength=len(K))
+    n1 = np.bincount(blk[req == 1], minlength=len(K))
+    n0p = np.where(n0 > 0, np.minimum(K, _cdiv(n0, 4) * 4), 0)
+    rem1 = np.maximum(0, n0 + n1 - n0p)
+    left = K - n0p
+    n1p = np.where(rem1 > 0, np.minimum(left, _cdiv(rem1, 8) * 8), 0)
+    n2p = left - n1p
+    up = (n2p > 0) & (n2p <= 8)
+    n1p, n2p = np.where(up, n1p + n2p, n1p), np.where(up, 0, n2p)
+    up = (n2p == 0) & (n1p > 0) & (n1p <= 4) & (n0p % 4 == 0)
+    n0p, n1p = np.where(up, n0p + n1p, n0p), np.where(up, 0, n1p)
+    order = np.lexsort((-w, blk))                      # stable: block by block, largest weight first
+    rank = np.empty(len(blk), np.int64)
+    rank[order] = np.arange(len(blk)) - first
+    return np.where(rank < n0p[blk], 0, np.where(rank < (n0p + n1p)[blk], 1, 2)).astype(np.int32)
+
+
+def class_counts(cls, offs):
+    """Terms per (block, pass, class) of classes in task order."""
+    task = np.repeat(np.arange(len(offs) - 1), np.diff(offs))
+    return np.bincount(3 * task + cls[:len(task)], minlength=3 * (len(offs) - 1)).reshape(-1, 2, 3)
+
+
 def build_plan_arrays_mixed(struct, dense_recs, cls_lists, dense_chunk=16, v_chunk=32, u_rows=512, stream=False,
-                            ncta=148, nwarps=None):
+                            ncta=148, nwarps=None, counts=None):
     """Work items, slot layout and packing records of the mixed storage (code 3):
     FP32 dense items as in the FP32 plan; per low-rank block and term class c
     (FP32, FP16, INT8) the class's own U / V arrays with column groups MIXED_CW[c].
-    cls_lists[bi] = (cls_S, cls_D) from classify_terms.  Pure numpy.
+    cls_lists[bi] = (cls_S, cls_D) from classify_terms, or counts[bi, pass, class] terms
+    of each class (class_counts).  Pure numpy.
 
     stream=True lays the work out for the persistent bulk-copy kernel k_stream:
     StreamTask lists of phase A (dense tasks of at most STREAM_DENSE_ROWS rows and
@@ -398,73 +459,58 @@ def build_plan_arrays_mixed(struct, dense_recs, cls_lists, dense_chunk=16, v_chu
     one TGather record per low-rank block (the t it gathers into tfull)."""
     if stream:
         return _build_stream_mixed(struct, dense_recs, cls_lists, ncta)
-    ditems, slot_rows, slot = _dense_items(dense_recs, 4, dense_recs["off32"], dense_chunk)
-    aca_blocks = [b for b in struct.blocks if b.aca]
-    u_off, v_off = [0, 0, 0], [0, 0, 0]
-    tp = sb = 0
-    vitems, utasks, pack = [], [], []
-    lr_bytes = 0
-    kmax = 0
-    counts = np.zeros((3, 2), np.int64)      # terms per (class, slip)
-    vgroups = {}                             # (column start, columns, class) -> the blocks' V rows
-    for bi, b in enumerate(aca_blocks):
-        m, nn = len(b.row.indices), len(b.col.indices)
-        lo, hi = getattr(b, "rows", (0, m))
-        cS, cD = cls_lists[bi]
-        ks = np.bincount(cS, minlength=3).tolist()
-        kd = np.bincount(cD, minlength=3).tolist()
-        if sum(ks) + sum(kd) == 0:
-            continue
-        Ks = [_cdiv(ks[c] + kd[c], MIXED_CW[c]) * MIXED_CW[c] for c in range(3)]
-        Qs = [3 * (ks[c] + kd[c]) for c in range(3)]
-        kmax = max(kmax, sum(Ks))
-        rec_off, rec_tp, rec_nch, rec_sb, rec_voff = [0] * 3, [0] * 3, [0] * 3, [0] * 3, [0] * 3
-        for c in range(3):
-            counts[c] += (ks[c], kd[c])
-            cw = MIXED_CW[c]
-            lr_bytes += Qs[c] * ((hi - lo) + nn) * MIXED_BYTES[c] + (Qs[c] * 4 if c else 0)
-            rec_off[c], rec_voff[c] = u_off[c], v_off[c]
-            if Ks[c] == 0:
-                continue
-            lead = b.col.start % cw
-            ngv = _cdiv(nn + lead, cw)
-            gch = min(v_chunk, _lib.STREAM_XMAX // cw) if stream else v_chunk
-            nch = _cdiv(ngv, gch)
-            if stream and Qs[c] * 16 > _lib.STREAM_STAGE_BYTES:
-                raise _lib.Pq3dError("a block's term class has %d V rows, more than one stream stage holds" % Qs[c])
-            if stream:
-                for ch in range(nch):
-                    g0, g1 = ch * gch, min(ngv, (ch + 1) * gch)
-                    vitems.append((v_off[c], Qs[c], 0, Qs[c], g0, g1, b.col.start - lead, (3 * ks[c]) | (c << 16),
-                                   tp + ch * Qs[c]))
-            else:
-                # the block's V rows join those of the other blocks with the same columns
-                vgroups.setdefault((b.col.start, nn, c), []).append((v_off[c], Qs[c], 3 * ks[c], tp))
-            rec_tp[c], rec_nch[c] = tp, nch
-            tp += nch * Qs[c]
-            if c:
-                rec_sb[c] = sb
-                sb += Qs[c]
-            u_off[c] += Ks[c] * m * 3
-            v_off[c] += Qs[c] * ngv * cw
-        for r0 in range(lo, hi, u_rows):
-            utasks.append((rec_off, m, r0, min(hi, r0 + u_rows), slot - lo, Ks, ks, kd, Qs, rec_tp, rec_nch, rec_sb, 0))
-        slot_rows.append((slot, b.row.start + lo, hi - lo))
-        for p in (0, 1):
-            pack.append((bi, p, rec_off, rec_voff, ks, kd, Qs, Ks, rec_sb))
-        slot += hi - lo
+    ditems, slot_rows, slot0 = _dense_items(dense_recs, 4, dense_recs["off32"], dense_chunk)
+    if counts is None:
+        counts = np.array([[np.bincount(c, minlength=3) for c in cl] for cl in cls_lists], np.int64).reshape(-1, 2, 3)
+    CW = np.array(MIXED_CW)
+    m, nn, row0, c0, lo, hi = _block_geometry([b for b in struct.blocks if b.aca])
+    on = np.nonzero(counts.sum(axis=(1, 2)) > 0)[0]              # blocks with terms
+    m, nn, row0, c0, lo, hi = (a[on] for a in (m, nn, row0, c0, lo, hi))
+    ks, kd = counts[on, 0], counts[on, 1]                        # (block, class)
+    K = _cdiv(ks + kd, CW) * CW
+    Q = 3 * (ks + kd)
+    lead = c0[:, None] % CW
+    ngv = _cdiv(nn[:, None] + lead, CW)
+    nch = np.where(K > 0, _cdiv(ngv, v_chunk), 0)
+    # class arrays one after the other within a class; partials and scales over (block, class)
+    u_off, v_off, u_size, v_size = np.zeros_like(K), np.zeros_like(K), [], []
+    for c in range(3):
+        u_off[:, c], t = _offsets(K[:, c] * m * 3)
+        u_size.append(t)
+        v_off[:, c], t = _offsets(Q[:, c] * ngv[:, c] * MIXED_CW[c])
+        v_size.append(t)
+    if max(v_size) >= 1 << 32:
+        raise _lib.Pq3dError("a V class array of the mixed storage holds 2^32 elements or more")
+    tp, n_tpart = _offsets((nch * Q).ravel())
+    scaled = np.where(np.arange(3) > 0, Q, 0).ravel()
+    sb, n_scales = _offsets(scaled)
+    tp, sb = np.where(K > 0, tp.reshape(-1, 3), 0), np.where((K > 0) & (np.arange(3) > 0), sb.reshape(-1, 3), 0)
+    slot, n_slots = _offsets(hi - lo)
+    slot, n_slots = slot + slot0, n_slots + slot0
+    # one entry per (block, class) with rows, for the merged V items
+    b, c = np.nonzero(K > 0)
+    vitems, vwarp, vrows = _merged_v_items(c0[b], nn[b], c, v_off[b, c], Q[b, c], 3 * ks[b, c], tp[b, c], v_chunk,
+                                           nwarps or VMIX_WARPS)
+    o, i = _expand(_cdiv(hi - lo, u_rows))
+    r0 = lo[o] + i * u_rows
+    nu = len(o)
+    utasks = _fields(_lib.U_TASK_M, nu, off=u_off[o], m=m[o], r0=r0, r1=np.minimum(hi[o], r0 + u_rows),
+                     slot=(slot - lo)[o], K=K[o], kS=ks[o], kD=kd[o], Q=Q[o], tp=tp[o], nch=nch[o], sb=sb[o])
+    slot_rows = np.concatenate([slot_rows, np.stack([slot, row0 + lo, hi - lo], axis=1)])
+    pack = np.zeros(2 * len(on), dtype=_PACK_M)
+    for k, v in dict(bi=on, u_off=u_off, v_off=v_off, kS=ks, kD=kd, Q=Q, K=K, sb=sb).items():
+        pack[k] = np.repeat(v, 2, axis=0)
+    pack["pass_"] = np.tile([0, 1], len(on))
     A = _leaf_lists(struct, slot_rows)
     dense_entries = int(np.sum(dense_recs["m"].astype(np.int64) * dense_recs["n"])) if len(dense_recs) else 0
     n = struct.n
-    vrows = vwarp = None
-    if not stream:
-        if max(v_off) >= 1 << 32:
-            raise _lib.Pq3dError("a V class array of the mixed storage holds 2^32 elements or more")
-        vitems, vwarp, vrows = _merged_v_items(vgroups, v_chunk, nwarps or VMIX_WARPS)
-    A.update(ditems=_rec(ditems, _lib.DENSE_ITEM), vitems=_rec(vitems, _lib.V_ITEM_M if not stream else _lib.V_ITEM),
-             vrows=vrows, vwarp=vwarp, utasks=_rec(utasks, _lib.U_TASK_M), n_ditems=len(ditems), n_vitems=len(vitems), n_utasks=len(utasks),
-             n_slots=slot, n_tpart=tp, n_scales=sb, kmax=kmax, u_sizes=u_off, v_sizes=v_off, pack=pack, stream=stream,
-             class_terms=counts, alg_bytes=dense_entries * 6 * 4 + lr_bytes + 2 * n * 4 + 3 * n * 8)
+    lr_bytes = int((Q * ((hi - lo) + nn)[:, None] * np.array(MIXED_BYTES)).sum() + 4 * scaled.sum())
+    nd = len(ditems)
+    A.update(ditems=_fields(_lib.DENSE_ITEM, 0) if nd == 0 else ditems, vitems=vitems, vrows=vrows, vwarp=vwarp,
+             utasks=utasks, n_ditems=nd, n_vitems=int(vwarp[-1]), n_utasks=nu, n_slots=n_slots, n_tpart=n_tpart,
+             n_scales=n_scales, kmax=int(K.sum(axis=1).max()) if len(K) else 0, u_sizes=u_size, v_sizes=v_size,
+             pack=pack, stream=False, class_terms=np.stack([ks.sum(axis=0), kd.sum(axis=0)], axis=1),
+             alg_bytes=dense_entries * 6 * 4 + lr_bytes + 2 * n * 4 + 3 * n * 8)
     return A
 
 
@@ -472,57 +518,63 @@ VMIX_WARPS = 8 * 148 * 4      # k_v_mixed warps when no device says otherwise (B
 VMIX_ROWS = 32                # rows per merged V item (k_v_mixed handles up to 32)
 
 
-def _merged_v_items(vgroups, v_chunk, nwarps=VMIX_WARPS):
+def _merged_v_items(col0, nn, cls, off, Q, ks3, tp, v_chunk, nwarps=VMIX_WARPS):
     """V items of the mixed storage's plain kernels (k_v_mixed): for each column
     cluster, class and slip, the V rows of all low-rank blocks with those columns
     (in block order), per column chunk, 32 rows to an item, so the x slice is loaded
-    once for all of them.  vgroups: (column start, columns, class) -> [(V offset of
-    the block in its class array, Q, strike rows, t base)].  Returns the items
+    once for all of them.  One entry per (block, class): column start, columns, class,
+    V offset in the class array, Q, strike rows, t base.  Returns the items
     ordered by warp, the per-warp offsets (nwarps + 1) and the row records.  Items go
     largest first to the least loaded of the nwarps warps (cost: row slots of 8 x
     column groups, plus a fixed start), so the persistent warps end together."""
-    items, recs = [], []
-    nrec = 0
-    for (col0, nn, c), blocks in vgroups.items():
-        cw = MIXED_CW[c]
-        lead = col0 % cw
-        ngv = _cdiv(nn + lead, cw)
-        nch = _cdiv(ngv, v_chunk)
-        bl = np.array(blocks, dtype=np.int64).reshape(-1, 4)     # off, Q, strike rows, t base
-        for s_ in (0, 1):
-            # the slip's rows of every block, in block order: q in [0, ks3) or [ks3, Q)
-            lo = np.zeros(len(bl), np.int64) if s_ == 0 else bl[:, 2]
-            cnt = (bl[:, 2] if s_ == 0 else bl[:, 1]) - lo
-            nrows = int(cnt.sum())
-            if nrows == 0:
-                continue
-            blk = np.repeat(np.arange(len(bl)), cnt)
-            q = np.arange(nrows) - np.repeat(np.cumsum(cnt) - cnt, cnt) + lo[blk]
-            off, Q, tp = bl[blk, 0], bl[blk, 1], bl[blk, 3]
-            for ch in range(nch):
-                g0, g1 = ch * v_chunk, min(ngv, (ch + 1) * v_chunk)
-                for r in range(0, nrows, VMIX_ROWS):
-                    items.append((nrec + r, min(VMIX_ROWS, nrows - r), g0, g1, col0 - lead, s_ | (c << 8), 0))
-                # row records of this chunk's items, consecutive in item order
-                recs.append(np.stack([off + q * cw, Q * cw, tp + ch * Q + q], axis=1))
-                nrec += nrows
+    # entries grouped by (columns, class), groups in order of first appearance
+    _, first, grp = np.unique(np.stack([col0, nn, cls], axis=1), axis=0, return_index=True, return_inverse=True)
+    grp = np.argsort(np.argsort(first))[grp.ravel()]
+    e = np.argsort(grp, kind="stable")
+    grp, off, Q, ks3, tp = grp[e], off[e], Q[e], ks3[e], tp[e]
+    g0 = np.sort(first)                                          # a group's first entry
+    col0, nn, cls = col0[g0], nn[g0], cls[g0]
+    cw = np.array(MIXED_CW)[cls]
+    lead = col0 % cw
+    ngv = _cdiv(nn + lead, cw)
+    nch = _cdiv(ngv, v_chunk)
+    ng = len(g0)
+    # rows of group g, slip s: q in [0, ks3) or [ks3, Q) of its entries, in order
+    cnt = np.stack([ks3, Q - ks3], axis=1)
+    eo = np.lexsort((np.tile(np.arange(len(grp)), 2), np.concatenate([2 * grp, 2 * grp + 1])))
+    ent, slip = eo % max(len(grp), 1), eo // max(len(grp), 1)
+    o, q = _expand(cnt[ent, slip])
+    ent, slip = ent[o], slip[o]
+    q = q + np.where(slip == 1, ks3[ent], 0)
+    gs = 2 * grp[ent] + slip                                     # sorted: rows of (group, slip) are consecutive
+    nrows = np.bincount(gs, minlength=2 * ng)
+    row0, _ = _offsets(nrows)
+    # per (group, slip, chunk): the rows' records, then its items of 32 rows
+    a, ch = _expand(np.where(nrows > 0, np.repeat(nch, 2), 0))
+    rec0, nrec = _offsets(nrows[a])
+    o, i = _expand(nrows[a])
+    r = row0[a[o]] + i
+    rec = _fields(_lib.V_ROW, nrec, base=off[ent[r]] + q[r] * cw[grp[ent[r]]], stride=Q[ent[r]] * cw[grp[ent[r]]],
+                  out=tp[ent[r]] + ch[o] * Q[ent[r]] + q[r])
+    o, i = _expand(_cdiv(nrows[a], VMIX_ROWS))
+    g = a[o] // 2
+    nitems = len(o)
+    items = _fields(_lib.V_ITEM_M, nitems, rows=rec0[o] + VMIX_ROWS * i, nr=np.minimum(VMIX_ROWS, nrows[a[o]] - VMIX_ROWS * i),
+                    g0=ch[o] * v_chunk, g1=np.minimum(ngv[g], (ch[o] + 1) * v_chunk), c0=(col0 - lead)[g],
+                    s=a[o] % 2 | (cls[g] << 8))
     import heapq
-    cost = [((nr + 7) // 8) * (g1 - g0) + 16 for _, nr, g0, g1, _, _, _ in items]
-    order = sorted(range(len(items)), key=lambda i: -cost[i])
-    nwarps = max(8, min(int(nwarps), max(len(items), 1)) // 8 * 8)
+    it = items[:nitems]
+    cost = _cdiv(it["nr"], 8) * (it["g1"] - it["g0"]) + 16
+    order = np.argsort(-cost, kind="stable")
+    nwarps = max(8, min(int(nwarps), max(nitems, 1)) // 8 * 8)
     heap = [(0, w) for w in range(nwarps)]
-    lists = [[] for _ in range(nwarps)]
-    for i in order:
-        load, w = heapq.heappop(heap)
-        lists[w].append(i)
-        heapq.heappush(heap, (load + cost[i], w))
-    vwarp = np.zeros(nwarps + 1, dtype=np.int32)
-    vwarp[1:] = np.cumsum([len(l) for l in lists])
-    items = [items[i] for l in lists for i in l]
-    rec = np.zeros(max(nrec, 1), dtype=_lib.V_ROW)
-    if recs:
-        a = np.concatenate(recs)
-        rec["base"], rec["stride"], rec["out"] = a[:, 0], a[:, 1], a[:, 2]
+    warp = np.empty(nitems, np.int32)
+    for k, c in enumerate(cost[order].tolist()):
+        load, w = heap[0]
+        warp[k] = w
+        heapq.heapreplace(heap, (load + c, w))
+    vwarp = np.concatenate([[0], np.cumsum(np.bincount(warp, minlength=nwarps))]).astype(np.int32)
+    items[:nitems] = it[order[np.argsort(warp, kind="stable")]]
     return items, vwarp, rec
 
 
@@ -778,7 +830,7 @@ class DeviceHMatrix:
         self.assembled = True
         if not self.keep_factors:
             # packed copies are all that the matvec needs: release the FP64 ACA workspaces
-            self.aca_ws = [(None, keep) for _, keep in self.aca_ws]
+            self.aca_ws = [None] * len(self.aca_ws)
             torch.cuda.empty_cache()
         return self
 
@@ -804,86 +856,64 @@ class DeviceHMatrix:
         starts = getattr(self.s, "aca_starts", None)
         if starts is None:
             starts = aca_start_indices(self.s.blocks, self.aca_seed)
-        rowlist, collist = [], []
-        tasks = []
-        roff = 0
-        for bi, b in enumerate(self.aca_blocks):
-            m, n = len(b.row.indices), len(b.col.indices)
-            rowlist.append(b.row.indices)
-            collist.append(b.col.indices)
-            for p in (0, 1):
-                tasks.append(dict(block=bi, pass_=p, m=m, n=n, rows_off=roff, cols_off=roff,
-                                  iref0=starts[bi][p][0], jref0=starts[bi][p][1]))
-            roff += 0  # offsets assigned below
-        # row and col lists stored separately
-        rl = np.concatenate(rowlist).astype(np.int32) if rowlist else np.zeros(1, np.int32)
-        cl = np.concatenate(collist).astype(np.int32) if collist else np.zeros(1, np.int32)
-        ro = np.concatenate([[0], np.cumsum([len(r) for r in rowlist])]).astype(np.int64) if rowlist else np.zeros(1, np.int64)
-        co = np.concatenate([[0], np.cumsum([len(c) for c in collist])]).astype(np.int64) if collist else np.zeros(1, np.int64)
-        for t in tasks:
-            t["rows_off"] = int(ro[t["block"]])
-            t["cols_off"] = int(co[t["block"]])
-        self.rowlist = torch.tensor(rl, dtype=torch.int32, device=self.dev)
-        self.collist = torch.tensor(cl, dtype=torch.int32, device=self.dev)
-        self.aca_tasks = tasks
-        self.aca_ranks = np.zeros(len(tasks), dtype=np.int32)
-        self.aca_flags = np.zeros(len(tasks), dtype=np.int32)
-        self.aca_ws = []  # (tensor, {task index: ws_off, kmax})
-        pending = list(range(len(tasks)))
-        kcap = self.kcap
-        while pending:
+        blocks = self.aca_blocks
+        nt = 2 * len(blocks)                     # tasks: strike and dip pass of every block
+        m, n = (np.repeat(v, 2) for v in _block_geometry(blocks)[:2])
+        start = np.array(starts, dtype=np.int64).reshape(-1, 2)
+        none = [np.zeros(1, np.int32)]           # row and column lists stored separately
+        self.rowlist = torch.from_numpy(np.concatenate([b.row.indices for b in blocks] or none).astype(np.int32)).to(self.dev)
+        self.collist = torch.from_numpy(np.concatenate([b.col.indices for b in blocks] or none).astype(np.int32)).to(self.dev)
+        ro, co = self._row_offsets()
+        self.aca_ranks = np.zeros(nt, dtype=np.int32)
+        self.aca_flags = np.zeros(nt, dtype=np.int32)
+        self.aca_ws = []                         # workspaces; a task's is task_ws["ws"][task]
+        self.task_ws = {k: np.zeros(nt, np.int64) for k in ("ws", "off", "kmax")}
+        kcap = np.minimum(np.minimum(m, n), self.kcap)
+        pending = np.arange(nt)
+        while len(pending):
             # batches bounded by the workspace budget, largest tasks first
-            pending.sort(key=lambda i: -(tasks[i]["m"] + tasks[i]["n"]))
+            pending = pending[np.argsort(-(m + n)[pending], kind="stable")]
             retry = []
             i0 = 0
             while i0 < len(pending):
-                batch, ws_off = [], 0
-                while i0 < len(pending):
-                    t = tasks[pending[i0]]
-                    kmax = min(t["m"], t["n"], t.get("kcap", kcap))
-                    need = self.L.pq3d_aca_ws_doubles(t["m"], t["n"], kmax)
-                    if batch and (ws_off + need) * 8 > self.ws_budget:
-                        break
-                    batch.append((pending[i0], ws_off, kmax))
-                    ws_off += need
-                    i0 += 1
-                rec = np.zeros(len(batch), dtype=_lib.ACA_TASK)
-                max_mn = 0
-                for j, (ti, wo, kmax) in enumerate(batch):
-                    t = tasks[ti]
-                    rec[j] = (t["rows_off"], t["cols_off"], wo, t["m"], t["n"], kmax, t["pass_"], t["iref0"], t["jref0"])
-                    max_mn = max(max_mn, t["m"], t["n"])
-                ws = torch.empty(max(ws_off, 1), dtype=torch.float64, device=self.dev)
+                t = pending[i0:]
+                end = np.cumsum(3 * kcap[t] * (m[t] + n[t]) + 6 * (m[t] + n[t]))        # pq3d_aca_ws_doubles
+                t = t[:max(1, int(np.searchsorted(end * 8, self.ws_budget, side="right")))]
+                end = end[:len(t)]
+                i0 += len(t)
+                rec = np.zeros(len(t), dtype=_lib.ACA_TASK)
+                for k, v in dict(rows_off=ro[t // 2], cols_off=co[t // 2], ws_off=np.concatenate([[0], end[:-1]]), m=m[t],
+                                 n=n[t], kmax=kcap[t], pass_=t % 2, iref0=start[t, 0], jref0=start[t, 1]).items():
+                    rec[k] = v
+                if int(end[0]) != self.L.pq3d_aca_ws_doubles(int(m[t[0]]), int(n[t[0]]), int(kcap[t[0]])):
+                    raise _lib.Pq3dError("ACA workspace layout mismatch")
+                max_mn = int(max(m[t].max(), n[t].max()))
+                ws = torch.empty(int(end[-1]), dtype=torch.float64, device=self.dev)
                 d_rec = torch.from_numpy(rec.view(np.uint8)).to(self.dev)
-                d_rank = torch.zeros(len(batch), dtype=torch.int32, device=self.dev)
-                d_flag = torch.zeros(len(batch), dtype=torch.int32, device=self.dev)
+                d_out = torch.zeros((2, len(t)), dtype=torch.int32, device=self.dev)      # ranks, flags
                 check(self.L.pq3d_aca_batched(ptr(self.xg), ptr(self.ev), ptr(self.rec), ptr(self.rowlist),
-                                              ptr(self.collist), ptr(d_rec), len(batch), ptr(ws), self.mu, self.lam,
-                                              self.aca_tol, 1 if self.aca_rel else 0, max_mn, ptr(d_rank),
-                                              ptr(d_flag), ptr(self.hs), self.halfspace, self._stream),
+                                              ptr(self.collist), ptr(d_rec), len(t), ptr(ws), self.mu, self.lam,
+                                              self.aca_tol, 1 if self.aca_rel else 0, max_mn, ptr(d_out[0]),
+                                              ptr(d_out[1]), ptr(self.hs), self.halfspace, self._stream),
                       "pq3d_aca_batched")
-                ranks = d_rank.cpu().numpy()
-                flags = d_flag.cpu().numpy()
+                ranks, flags = d_out.cpu().numpy()
                 if (flags & 8).any():
                     raise _lib.Pq3dError("pq3d_aca_batched: a task has more rows or columns than the batch's "
                                          "max_mn (not run)")
                 # flag 4 (every remaining pivot candidate excluded) ends a task normally: the
                 # factors found so far are the block's approximation, as in the reference loop
-                keep = {}
-                for j, (ti, wo, kmax) in enumerate(batch):
-                    if flags[j] & 1 and kmax < min(tasks[ti]["m"], tasks[ti]["n"]):
-                        tasks[ti]["kcap"] = min(2 * kmax, min(tasks[ti]["m"], tasks[ti]["n"]))
-                        retry.append(ti)
-                        continue
-                    self.aca_ranks[ti] = ranks[j]
-                    self.aca_flags[ti] = flags[j]
-                    keep[ti] = (wo, kmax)
-                self.aca_ws.append((ws, keep))
-            pending = retry
-        self.task_ws = {}
-        for wi, (ws, keep) in enumerate(self.aca_ws):
-            for ti, (wo, kmax) in keep.items():
-                self.task_ws[ti] = (wi, wo, kmax)
+                full = np.minimum(m[t], n[t])
+                again = (flags & 1 != 0) & (kcap[t] < full)
+                done = t[~again]
+                self.aca_ranks[done] = ranks[~again]
+                self.aca_flags[done] = flags[~again]
+                self.task_ws["ws"][done] = len(self.aca_ws)
+                self.task_ws["off"][done] = rec["ws_off"][~again]
+                self.task_ws["kmax"][done] = kcap[done]
+                self.aca_ws.append(ws)
+                kcap[t[again]] = np.minimum(2 * kcap[t], full)[again]
+                retry.append(t[again])
+            pending = np.concatenate(retry)
 
     def ranks(self):
         """(kS, kD) per ACA block."""
@@ -906,21 +936,14 @@ class DeviceHMatrix:
         Ubuf = torch.zeros(max(A["u_size"], 8), dtype=lr_dtype, device=self.dev)
         Vbuf = torch.zeros(max(A["v_size"], 8), dtype=lr_dtype, device=self.dev)
         # pack every ACA task into the layout, one launch per workspace batch
-        ro_np = self._row_offsets()
-        by_ws = {}
-        for (bi, p, u_off, v_off, K, Q, ks, kd) in A["pack"]:
-            ti = 2 * bi + p
-            wi, wo, kmax = self.task_ws[ti]
-            b = self.aca_blocks[bi]
-            by_ws.setdefault(wi, []).append((wo, u_off, v_off, ro_np[bi][0], ro_np[bi][1], len(b.row.indices),
-                                             len(b.col.indices), kmax, ks if p == 0 else kd, p, ks, kd, K, Q,
-                                             b.row.start, b.col.start, 1 if self.aca_flags[ti] & 2 else 0))
-        for wi, rows in by_ws.items():
-            rec = np.array(rows, dtype=_lib.PACK_TASK)
-            d_rec = torch.from_numpy(rec.view(np.uint8)).to(self.dev)
-            check(self.L.pq3d_aca_pack(ptr(d_rec), len(rows), ptr(self.aca_ws[wi][0]), ptr(self.rowlist),
-                                       ptr(self.collist), ptr(self.iperm), code, ptr(Ubuf), ptr(Vbuf), self._stream),
-                  "pq3d_aca_pack")
+        K = A["pack"]
+        ti = 2 * K["bi"] + K["pass_"]
+        rec = self._task_records(_lib.PACK_TASK, ti)
+        for k in ("u_off", "v_off", "kS", "kD", "K", "Q"):
+            rec[k] = K[k]
+        for wi, d_rec, k in self._by_workspace(rec, ti):
+            check(self.L.pq3d_aca_pack(ptr(d_rec), k, ptr(self.aca_ws[wi]), ptr(self.rowlist), ptr(self.collist),
+                                       ptr(self.iperm), code, ptr(Ubuf), ptr(Vbuf), self._stream), "pq3d_aca_pack")
         return self._finish_plan(dtype, A, Ubuf, Vbuf)
 
     def shapes(self, dtype):
@@ -947,10 +970,7 @@ class DeviceHMatrix:
             return None
         if DTYPES[dtype] == 3:
             offs = np.concatenate([[0], np.cumsum(np.asarray(self.aca_ranks, np.int64))])
-            t = self.mixed_tmap
-            cls_lists = [(t[offs[2 * bi]:offs[2 * bi + 1]] & 3, t[offs[2 * bi + 1]:offs[2 * bi + 2]] & 3)
-                         for bi in range(len(self.aca_blocks))]
-            A = self._mixed_arrays(cls_lists)
+            A = self._mixed_arrays(self.mixed_tmap & 3, offs)
             A["mixed"] = P["mixed"]
         else:
             A = self.plan_arrays(dtype)
@@ -965,26 +985,22 @@ class DeviceHMatrix:
         dc, vc, ur = self.shapes(dtype)
         return build_plan_arrays(self.s, self.dense_recs, kS, kD, code, dc, vc, ur)
 
-    def _task_records_mixed(self, keep_ws):
-        """PackTaskM records (per workspace batch) for every ACA task, with the weight /
-        term-map offset of each task (tasks in block order, strike pass first)."""
-        ro_np = self._row_offsets()
-        recs, tmap_off = {}, 0
-        offs = np.zeros(len(self.aca_tasks) + 1, np.int64)
-        for ti in range(len(self.aca_tasks)):
-            bi, p = divmod(ti, 2)
-            k = int(self.aca_ranks[ti])
-            offs[ti] = tmap_off
-            wi, wo, kmax = self.task_ws[ti]
-            b = self.aca_blocks[bi]
-            r = np.zeros(1, dtype=_lib.PACK_TASK_M)
-            r["ws_off"], r["rows_off"], r["cols_off"], r["tmap_off"] = wo, ro_np[bi][0], ro_np[bi][1], tmap_off
-            r["m"], r["n"], r["kmax"], r["k"], r["pass_"] = len(b.row.indices), len(b.col.indices), kmax, k, p
-            r["r0"], r["c0"], r["zeroB"] = b.row.start, b.col.start, 1 if self.aca_flags[ti] & 2 else 0
-            recs.setdefault(wi, []).append((ti, r))
-            tmap_off += k
-        offs[-1] = tmap_off
-        return recs, offs
+    def _task_records(self, dtype, ti):
+        """Pack records (PACK_TASK or PACK_TASK_M) of tasks ti: workspace, lists, sizes, rank."""
+        m, n, r0, c0, _, _ = (v[ti // 2] for v in _block_geometry(self.aca_blocks))
+        ro, co = (v[ti // 2] for v in self._row_offsets())
+        rec = np.zeros(len(ti), dtype=dtype)
+        for k, v in dict(ws_off=self.task_ws["off"][ti], rows_off=ro, cols_off=co, m=m, n=n, kmax=self.task_ws["kmax"][ti],
+                         k=self.aca_ranks[ti], pass_=ti % 2, r0=r0, c0=c0, zeroB=self.aca_flags[ti] & 2 != 0).items():
+            rec[k] = v
+        return rec
+
+    def _by_workspace(self, rec, ti):
+        """(workspace, records on the device, their number) per workspace batch."""
+        ws = self.task_ws["ws"][ti]
+        for wi in np.unique(ws):
+            r = rec[ws == wi]
+            yield int(wi), self.torch.from_numpy(r.view(np.uint8)).to(self.dev), len(r)
 
     def _plan_mixed(self):
         """Mixed storage (code 3): FP32 dense near field; ACA terms in FP32 / FP16 / INT8
@@ -1003,29 +1019,25 @@ class DeviceHMatrix:
             check(L.pq3d_nearfield_rowabs(ptr(self.dense32), ptr(d_recs), len(recs), n, ptr(R3), st),
                   "pq3d_nearfield_rowabs")
         R = R3.view(3, n).max(dim=0).values.contiguous()
-        by_ws, offs = self._task_records_mixed(None)
+        # every task's weights, and the offset of its terms (tasks in block order, strike first)
+        tasks = np.arange(2 * len(self.aca_blocks))
+        offs = np.concatenate([[0], np.cumsum(self.aca_ranks, dtype=np.int64)])
+        rec = self._task_records(_lib.PACK_TASK_M, tasks)
+        rec["tmap_off"] = offs[:-1]
         w = torch.zeros(max(int(offs[-1]), 1), dtype=torch.float64, device=self.dev)
-        for wi, rows in by_ws.items():
-            rec = np.concatenate([r for _, r in rows])
-            d_rec = torch.from_numpy(rec.view(np.uint8)).to(self.dev)
-            check(L.pq3d_aca_term_weights(ptr(d_rec), len(rec), ptr(self.aca_ws[wi][0]), ptr(self.rowlist),
-                                          ptr(self.iperm), ptr(R), ptr(w), st), "pq3d_aca_term_weights")
-        w = w.cpu().numpy()
-        # classes per block, then each term's position within its class (per pass)
-        tmap = np.zeros(max(int(offs[-1]), 1), np.int32)
-        cls_lists = []
-        for bi in range(len(self.aca_blocks)):
-            tS, tD = 2 * bi, 2 * bi + 1
-            cS, cD = classify_terms(w[offs[tS]:offs[tS + 1]], w[offs[tD]:offs[tD + 1]], self.mixed_tol)
-            cls_lists.append((cS, cD))
-            for ti, cc in ((tS, cS), (tD, cD)):
-                pos = np.zeros(len(cc), np.int32)
-                for c in range(3):
-                    sel = np.nonzero(cc == c)[0]
-                    pos[sel] = np.arange(len(sel))
-                tmap[offs[ti]:offs[ti + 1]] = cc | (pos << 2)
-        self.mixed_tmap = tmap[:int(offs[-1])]
-        A = self._mixed_arrays(cls_lists)
+        for wi, d_rec, k in self._by_workspace(rec, tasks):
+            check(L.pq3d_aca_term_weights(ptr(d_rec), k, ptr(self.aca_ws[wi]), ptr(self.rowlist), ptr(self.iperm),
+                                          ptr(R), ptr(w), st), "pq3d_aca_term_weights")
+        # every term's class, and its position within its task's terms of that class
+        cls = classify_blocks(w.cpu().numpy()[:int(offs[-1])], offs, self.mixed_tol)
+        key = 3 * np.repeat(tasks, self.aca_ranks) + cls
+        order = np.argsort(key, kind="stable")
+        pos = np.empty(len(cls), np.int64)
+        pos[order] = _expand(np.bincount(key, minlength=3 * len(tasks)))[1]
+        tmap = np.zeros(max(len(cls), 1), np.int32)
+        tmap[:len(cls)] = cls | (pos << 2)
+        self.mixed_tmap = tmap[:len(cls)]
+        A = self._mixed_arrays(cls, offs)
         # INT8-class entries are stored as b + 128: the fill 128 decodes to zero, so padding
         # columns (a block's lead and tail columns, its K padding) contribute nothing
         tdt, fill = (torch.float32, torch.float16, torch.uint8), (0, 0, 128)
@@ -1033,51 +1045,43 @@ class DeviceHMatrix:
         Vb = [torch.full((max(int(A["v_sizes"][c]), 16),), fill[c], dtype=tdt[c], device=self.dev) for c in range(3)]
         scales = torch.zeros(max(A["n_scales"], 4), dtype=torch.float32, device=self.dev)
         d_tmap = torch.from_numpy(tmap).to(self.dev)
-        layout = {}
-        for (bi, p, uo, vo, ks, kd, Q, K, sb) in A["pack"]:
-            layout[2 * bi + p] = (uo, vo, ks, kd, Q, K, sb)
-        for wi, rows in by_ws.items():
-            recl = []
-            for ti, r in rows:
-                if ti not in layout:
-                    continue                       # a block without terms
-                uo, vo, ks, kd, Q, K, sb = layout[ti]
-                r = r.copy()
-                r["u_off"], r["v_off"], r["kS"], r["kD"], r["Q"], r["K"], r["sb"] = uo, vo, ks, kd, Q, K, sb
-                recl.append(r)
-            if not recl:
-                continue
-            rec = np.concatenate(recl)
-            d_rec = torch.from_numpy(rec.view(np.uint8)).to(self.dev)
-            check(L.pq3d_aca_pack_mixed(ptr(d_rec), len(rec), ptr(self.aca_ws[wi][0]), ptr(self.rowlist),
-                                        ptr(self.collist), ptr(self.iperm), ptr(d_tmap), ptr(Ub[0]), ptr(Ub[1]),
-                                        ptr(Ub[2]), ptr(Vb[0]), ptr(Vb[1]), ptr(Vb[2]), ptr(scales), st),
-                  "pq3d_aca_pack_mixed")
+        K = A["pack"]                              # blocks with terms
+        if self.mixed_stream and A.get("stream"):
+            K = np.array([tuple(k) for k in K], dtype=_PACK_M)
+        ti = 2 * K["bi"] + K["pass_"]
+        rec = rec[ti]
+        for k in ("u_off", "v_off", "kS", "kD", "Q", "K", "sb"):
+            rec[k] = K[k]
+        for wi, d_rec, k in self._by_workspace(rec, ti):
+            check(L.pq3d_aca_pack_mixed(ptr(d_rec), k, ptr(self.aca_ws[wi]), ptr(self.rowlist), ptr(self.collist),
+                                        ptr(self.iperm), ptr(d_tmap), ptr(Ub[0]), ptr(Ub[1]), ptr(Ub[2]), ptr(Vb[0]),
+                                        ptr(Vb[1]), ptr(Vb[2]), ptr(scales), st), "pq3d_aca_pack_mixed")
         A["mixed"] = dict(U=Ub, V=Vb, scales=scales, tol=self.mixed_tol, class_terms=A["class_terms"].tolist())
         return self._finish_plan("mixed", A, Ub[0], Vb[0])
 
-    def _mixed_arrays(self, cls_lists):
+    def _mixed_arrays(self, cls, offs):
+        """Plan arrays from every term's class (task order) and the tasks' term offsets."""
         dc, vc, ur = self.shapes("mixed")
         if self.mixed_stream:
             ncta = self.L.pq3d_stream_ctas()
             if ncta > 0:
                 try:
+                    cls_lists = [(cls[offs[i]:offs[i + 1]], cls[offs[i + 1]:offs[i + 2]])
+                                 for i in range(0, len(offs) - 1, 2)]
                     return build_plan_arrays_mixed(self.s, self.dense_recs, cls_lists, dc, vc, ur, stream=True,
                                                    ncta=ncta)
                 except _lib.Pq3dError:
                     pass               # a term class too large for a stream stage: the plain kernels
         nw = self.L.pq3d_vmix_ctas()
-        return build_plan_arrays_mixed(self.s, self.dense_recs, cls_lists, dc, vc, ur,
-                                       nwarps=8 * nw if nw > 0 else VMIX_WARPS)
+        return build_plan_arrays_mixed(self.s, self.dense_recs, None, dc, vc, ur,
+                                       nwarps=8 * nw if nw > 0 else VMIX_WARPS, counts=class_counts(cls, offs))
 
     def install_mixed(self, tmap, U, V, scales):
         """Register a mixed plan whose class arrays come from elsewhere (an operator
         checkpoint): tmap holds every term's class code (bits 0-1) in task order."""
         offs = np.concatenate([[0], np.cumsum(np.asarray(self.aca_ranks, np.int64))])
-        cls_lists = [(tmap[offs[2 * bi]:offs[2 * bi + 1]] & 3, tmap[offs[2 * bi + 1]:offs[2 * bi + 2]] & 3)
-                     for bi in range(len(self.aca_blocks))]
         self.mixed_tmap = np.asarray(tmap, np.int32)
-        A = self._mixed_arrays(cls_lists)
+        A = self._mixed_arrays(self.mixed_tmap & 3, offs)
         A["mixed"] = dict(U=list(U), V=list(V), scales=scales, tol=self.mixed_tol,
                           class_terms=A["class_terms"].tolist())
         return self._finish_plan("mixed", A, U[0], V[0])
@@ -1150,15 +1154,9 @@ class DeviceHMatrix:
         return P
 
     def _row_offsets(self):
-        if not hasattr(self, "_ro_cache"):
-            ro, co = 0, 0
-            res = []
-            for b in self.aca_blocks:
-                res.append((ro, co))
-                ro += len(b.row.indices)
-                co += len(b.col.indices)
-            self._ro_cache = res
-        return self._ro_cache
+        """Offsets of every ACA block's rows and columns in rowlist and collist."""
+        m, n = _block_geometry(self.aca_blocks)[:2]
+        return _offsets(m)[0], _offsets(n)[0]
 
     def kernel_status(self, dtype):
         """Status word of a plan's streamed kernels: 0, 1 after a timed-out wait, 2 after a
