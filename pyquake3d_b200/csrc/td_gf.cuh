@@ -34,8 +34,8 @@ __host__ __device__ inline double dot3(const double *a, const double *b)
     return a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
 }
 
-// Per-source setup (TDstressFS_C.cpp:294-385).
-__device__ inline void make_src_rec(const double *P1, const double *P2, const double *P3, SrcRec &s)
+// Per-source setup (TDstressFS_C.cpp:294-385), all but the angles, whose cosines it gives.
+__device__ inline void make_src_frame(const double *P1, const double *P2, const double *P3, SrcRec &s, double *cosines)
 {
     double vn[3];
     vn[0] = (P2[1] - P1[1]) * (P3[2] - P1[2]) - (P2[2] - P1[2]) * (P3[1] - P1[1]);
@@ -67,15 +67,25 @@ __device__ inline void make_src_rec(const double *P1, const double *P2, const do
         e12[j] /= n12; e13[j] /= n13; e23[j] /= n23;
         s.e12[j] = e12[j]; s.e13[j] = e13[j]; s.e23[j] = e23[j];
     }
-    double angA = acos(dot3(e12, e13));
-    double angB = acos((-e12[0]) * e23[0] + (-e12[1]) * e23[1] + (-e12[2]) * e23[2]);
-    double angC = acos(dot3(e23, e13));
-    double ang[3] = {angA, angB, angC};
-    for (int k = 0; k < 3; ++k) {
-        double a = -kPi + ang[k];
-        s.cA[k] = cos(a);
-        s.sA[k] = sin(a);
-    }
+    cosines[0] = dot3(e12, e13);
+    cosines[1] = (-e12[0]) * e23[0] + (-e12[1]) * e23[1] + (-e12[2]) * e23[2];
+    cosines[2] = dot3(e23, e13);
+}
+
+// cos and sin of (-pi + angle) for the dislocation at one vertex.
+__device__ inline void make_src_angle(double cosine, double &cA, double &sA)
+{
+    const double a = -kPi + acos(cosine);
+    cA = cos(a);
+    sA = sin(a);
+}
+
+__device__ inline void make_src_rec(const double *P1, const double *P2, const double *P3, SrcRec &s)
+{
+    double c[3];
+    make_src_frame(P1, P2, P3, s, c);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) make_src_angle(c[k], s.cA[k], s.sA[k]);
 }
 
 // Configuration of a TD-frame point (trimodefinder, TDstressFS_C.cpp:125-166).
