@@ -282,6 +282,22 @@ __device__ __forceinline__ void smem_vec<double, 2>(const double *p, double *o)
     o[0] = a.x; o[1] = a.y;
 }
 
+// Start bringing a U task's rows into L2: one bulk prefetch per column group and component
+// (rows [r0, r1), 16 B each).  They do not depend on the V partials the task waits for.  Used by
+// the FP32 tasks (product of 20,480 elements 137.9 -> 133.8 us, 9,000 61.9 -> 60.9, 60k 706 either
+// way); BF16 (20,480: 104.6 -> 106.5) and FP64 ones (60k: 1,438 -> 1,589) lose by it, and so does
+// every type when only the first wave's tasks prefetch.
+__device__ __forceinline__ void prefetch_u_rows(const void *U, int64_t off_bytes, int m, int r0, int r1, int ngroups,
+                                                int first, int stride)
+{
+    const int nb = (r1 - r0) * 16;
+    if (nb <= 0) return;
+    for (int e = first; e < 3 * ngroups; e += stride) {
+        const unsigned char *p = (const unsigned char *)U + off_bytes + ((int64_t)e * m + r0) * 16;
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(nb) : "memory");
+    }
+}
+
 template <typename TL, typename TA>
 __device__ __forceinline__ void u_task(const UTask &T, const TL *__restrict__ U, const TA *__restrict__ tpart,
                                        TA *__restrict__ slots, TA *ts)
@@ -340,58 +356,26 @@ k_du(const DenseItem *__restrict__ ditems, int64_t n_ditems, int64_t n_dblocks, 
         dense_v_item<TD, TL, TA>(w, ditems, n_ditems, nullptr, 0, D, nullptr, x, 0, slots, nullptr);
         return;
     }
+    const UTask T = tasks[blockIdx.x - n_dblocks];
+    if (std::is_same<TL, float>::value)
+        prefetch_u_rows(U, T.off * (int64_t)sizeof(TL), T.m, T.r0, T.r1, T.K * (int)sizeof(TL) / 16, threadIdx.x, blockDim.x);
     asm volatile("griddepcontrol.wait;" ::: "memory");
     extern __shared__ __align__(16) unsigned char smraw[];
-    const UTask T = tasks[blockIdx.x - n_dblocks];
     u_task<TL, TA>(T, U, tpart, slots, reinterpret_cast<TA *>(smraw));
 }
 
 
-// FP64 path: the U tasks as their own launch after k_dense_v (dense and V items
-// together), which measured faster at this precision than the split launch.
+// FP64 path: the U tasks as their own launch after k_dense_v (dense and V items together, which
+// measured faster at this precision than the split launch), in its tail: 20,480 elements 290 ->
+// 285 us, 9,000 120.5 -> 117.6 against a plain launch.
 template <typename TL, typename TA>
 __global__ void __launch_bounds__(256)
 k_u(const UTask *__restrict__ tasks, const TL *__restrict__ U, const TA *__restrict__ tpart, TA *__restrict__ slots)
 {
-    constexpr int CW = 16 / sizeof(TL);
     extern __shared__ __align__(16) unsigned char smraw[];
-    TA *ts = reinterpret_cast<TA *>(smraw);
     const UTask T = tasks[blockIdx.x];
-    for (int e = threadIdx.x; e < 3 * T.K; e += blockDim.x) {
-        const int c = e / T.K, q = e % T.K;
-        int row = -1;
-        if (q < T.kS) row = c * T.kS + q;
-        else if (q < T.kS + T.kD) row = 3 * T.kS + c * T.kD + (q - T.kS);
-        TA v = 0;
-        if (row >= 0)
-            v = sum_partials<TA>(tpart + T.tp + row, T.nch, T.Q);
-        ts[e] = v;
-    }
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int ng = T.K / CW;
-    const int64_t gstride = (int64_t)T.m * 3 * CW;   // one column group of U: 3 comps x m rows
-    for (int rb = T.r0 + warp * 32; rb < T.r1; rb += blockDim.x) {
-        const int r = rb + lane;
-        if (r >= T.r1) break;
-        TA acc[3] = {0, 0, 0};
-        const TL *p = U + T.off + (int64_t)r * CW;             // [group][comp][row][CW]
-        const int64_t cstride = (int64_t)T.m * CW;
-#pragma unroll 2
-        for (int g = 0; g < ng; ++g) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                Vec16<TL> d = ld_stream(p + c * cstride);
-                TA tv[CW];
-                smem_vec<TA, CW>(ts + c * T.K + g * CW, tv);
-#pragma unroll
-                for (int k = 0; k < CW; ++k) acc[c] += widen<TA>(d.v[k]) * tv[k];
-            }
-            p += gstride;
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) slots[3 * ((int64_t)T.slot + r) + c] = acc[c];
-    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    u_task<TL, TA>(T, U, tpart, slots, reinterpret_cast<TA *>(smraw));
 }
 
 // ------------------------------------------------------------------ mixed storage
@@ -1134,6 +1118,9 @@ k_rowsum(int n, int R, const int32_t *__restrict__ leaf_of_row, const int32_t *_
          const int32_t *__restrict__ leaf_off, const TA *__restrict__ slots, const double *__restrict__ add0,
          const double *__restrict__ add1, const double *__restrict__ add2, double *__restrict__ y)
 {
+    // A stage of the V-mode stepper may be launched while this one runs.  (Launching this one
+    // behind the U tasks in turn cost 2 to 7 us a product at 1,936 to 9,000 elements.)
+    asm volatile("griddepcontrol.launch_dependents;");
     const int64_t base = (int64_t)blockIdx.x * R;
     rowsum_rows<256>(slots, leaf_of_row, leaf_ptr, leaf_off, base, n, R, [&](int r, const double *v) {
         const int64_t i = base + r;
@@ -1225,8 +1212,18 @@ static int run_matvec(const HmPlan &P, const TA *x, TA *slots, TA *tpart, const 
             if (smem > 200 * 1024) return PQ3D_ERR_ARG;
             if (smem > 48 * 1024)
                 PQ3D_CHECK(cudaFuncSetAttribute(k_u<TL, TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            k_u<TL, TA><<<(unsigned)P.n_utasks, 256, smem, st>>>((const UTask *)P.utasks, (const TL *)P.U, tpart,
-                                                                 slots);
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)P.n_utasks);
+            cfg.blockDim = dim3(256);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = st;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[0].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = (P.n_vitems + nd_a) > 0 ? 1 : 0;
+            PQ3D_CHECK(cudaLaunchKernelEx(&cfg, k_u<TL, TA>, (const UTask *)P.utasks, (const TL *)P.U, (const TA *)tpart,
+                                          slots));
         }
     } else {
         const int64_t n_dblocks = (nd_b * 32 + 255) / 256;
@@ -1251,8 +1248,7 @@ static int run_matvec(const HmPlan &P, const TA *x, TA *slots, TA *tpart, const 
                                           (const TA *)tpart));
         }
     }
-    if (y)
-        launch_rowsum<TA>(P.n, P.leaf_of_row, P.leaf_ptr, P.leaf_off, slots, add0, add1, add2, y, st);
+    if (y) launch_rowsum<TA>(P.n, P.leaf_of_row, P.leaf_ptr, P.leaf_off, slots, add0, add1, add2, y, st);
     return pq3d_launch_status();
 }
 
@@ -1291,8 +1287,7 @@ static int run_matvec_mixed(const HmPlan &P, const float *x, float *slots, float
                                       (const __half *)P.U16, (const uint8_t *)P.U8, x, slots, (const float *)tpart,
                                       P.scales));
     }
-    if (y)
-        launch_rowsum<float>(P.n, P.leaf_of_row, P.leaf_ptr, P.leaf_off, slots, add0, add1, add2, y, st);
+    if (y) launch_rowsum<float>(P.n, P.leaf_of_row, P.leaf_ptr, P.leaf_off, slots, add0, add1, add2, y, st);
     return pq3d_launch_status();
 }
 
@@ -1331,8 +1326,7 @@ static int run_matvec_stream(const HmPlan &P, const float *x, float *slots, floa
         A.cta_ptr = P.cta_b;
         k_stream<<<(unsigned)P.ncta_b, ST_THREADS, sm, st>>>(A);
     }
-    if (y)
-        launch_rowsum<float>(P.n, P.leaf_of_row, P.leaf_ptr, P.leaf_off, slots, add0, add1, add2, y, st);
+    if (y) launch_rowsum<float>(P.n, P.leaf_of_row, P.leaf_ptr, P.leaf_off, slots, add0, add1, add2, y, st);
     return pq3d_launch_status();
 }
 

@@ -135,189 +135,177 @@ __device__ inline Solve vsolve(double tq, double sig, double psi, double a, doub
 {
     const double S = fabs(tq) / (a * sig);
     const double lk = log(2.0 * V0 * eta / (a * sig)) - psi / a;
-    double z;
+    double z = S;
     Solve r{0.0, 0, false};
-    bool ok;
-    // Undamped start z = S: one Newton step decides whether it is already the root (slow
-    // slip, negligible damping); the MLP is consulted only when it is not.
-    bool easy = false;
-    if (mode == 2 && P) {
+    bool solve = true, judged = false, network = false;
+    int cap = maxit;
+    if (mode >= 2 && P) {
+        // Undamped start z = S: its first Newton step (dz >= 0) decides whether it is already the
+        // root (slow slip, negligible damping).  Mode 2 consults the network when it is not, for
+        // at most 8 steps from its start.  Mode 3 takes the step and goes on with plain Newton
+        // when its correction is at most `gate` in z -- the usual case away from nucleation, where
+        // it converges in a step or two -- and only a larger one (strong radiation damping)
+        // evaluates the network.  The residual judges the network's solves, plain Newton from S is
+        // the fallback.
         const double e = exp(lk + S), q = exp(-2.0 * S);
         const double dz = 0.5 * e * (1.0 - q) / (1.0 + 0.5 * e * (1.0 + q));
-        easy = dz <= tol * fmax(1.0, S);
-    }
-    if (mode == 3 && P) {
-        // Gated network start.  The undamped start z = S takes its first Newton step
-        // (the "easy" test above); when that step's correction is at most `gate` in z
-        // the solve goes on with plain Newton from there -- the usual case away from
-        // nucleation, where it converges in a step or two -- and only a larger
-        // correction (strong radiation damping) evaluates the network, whose start Newton
-        // then refines.  The step from z = S counts as an iteration either way; the
-        // bracketed solve stays the fallback.
-        const double e0 = exp(lk + S), q0 = exp(-2.0 * S);
-        const double dz0 = 0.5 * e0 * (1.0 - q0) / (1.0 + 0.5 * e0 * (1.0 + q0));
-        r.iters = 1;
-        double z1 = S - dz0;
-        z1 = z1 < 0.0 ? 0.0 : z1;
-        if (dz0 <= tol * fmax(1.0, S)) {
-            z = S;
-        } else {
-            if (dz0 > gate) {
-                float f[5];
-                mlp_features(S, lk, a, b, sig, f);
-                z = S / (1.0 + exp(-(double)mlp_eval(P, f)));
-            } else {
-                z = z1;
-            }
-            ok = newton(S, lk, tol, maxit, z, r.iters);
-            const double e = exp(lk + z), res = fabs(z + 0.5 * e * (1.0 - exp(-2.0 * z)) - S);
-            if (!ok || res > 1e-10 * (1.0 + S)) {
-                r.fallback = true;
-                z = S;
-                ok = newton(S, lk, tol, maxit, z, r.iters);
-            }
+        solve = !(dz <= tol * fmax(1.0, S));
+        judged = solve;
+        network = solve && (mode == 2 || dz > gate);
+        if (mode == 3 || !solve) r.iters = 1;
+        if (mode == 2) cap = 8;
+        if (solve && !network) {
+            z = S - dz;
+            z = z < 0.0 ? 0.0 : z;
         }
-    } else if (mode == 2 && P && easy) {
-        z = S;
-        r.iters = 1;
-    } else if (mode == 2 && P) {
+    } else if (mode == 0 && Vprev != 0.0) {
+        const double L = log(fabs(Vprev) / (2.0 * V0)) + psi / a;
+        z = L > 20.0 ? L + 0.6931471805599453 : asinh(exp(L));
+        z = z < 0.0 ? 0.0 : (z > S ? S : z);
+    }
+    if (network) {
         float f[5];
         mlp_features(S, lk, a, b, sig, f);
-        const float q = mlp_eval(P, f);
-        z = S / (1.0 + exp(-(double)q));
-        // the MLP only proposes the start: a few Newton steps, judged by the residual
-        ok = newton(S, lk, tol, 8, z, r.iters);
-        const double e = exp(lk + z), res = fabs(z + 0.5 * e * (1.0 - exp(-2.0 * z)) - S);
-        if (!ok || res > 1e-10 * (1.0 + S)) {
-            r.fallback = true;
-            z = S;
-            ok = newton(S, lk, tol, maxit, z, r.iters);
-        }
-    } else {
-        if (mode == 0 && Vprev != 0.0) {
-            const double L = log(fabs(Vprev) / (2.0 * V0)) + psi / a;
-            z = L > 20.0 ? L + 0.6931471805599453 : asinh(exp(L));
-            z = z < 0.0 ? 0.0 : (z > S ? S : z);
-        } else {
-            z = S;
-        }
-        ok = newton(S, lk, tol, maxit, z, r.iters);
-        if (ok && logx && S > 0.0) {
-            const unsigned long long slot = atomicAdd(logn, 1ull);
-            if ((long long)slot < logcap) {
-                float *o = logx + 6 * slot;
-                mlp_features(S, lk, a, b, sig, o);
-                double ratio = z / S;
-                ratio = ratio < 1e-6 ? 1e-6 : (ratio > 1.0 - 1e-6 ? 1.0 - 1e-6 : ratio);
-                o[5] = (float)log(ratio / (1.0 - ratio));
-            }
-        }
+        z = S / (1.0 + exp(-(double)mlp_eval(P, f)));
     }
-    (void)ok;
+    while (solve) {
+        const bool ok = newton(S, lk, tol, cap, z, r.iters);
+        if (!judged) {
+            if (ok && logx && S > 0.0) {
+                const unsigned long long slot = atomicAdd(logn, 1ull);
+                if ((long long)slot < logcap) {
+                    float *o = logx + 6 * slot;
+                    mlp_features(S, lk, a, b, sig, o);
+                    double ratio = z / S;
+                    ratio = ratio < 1e-6 ? 1e-6 : (ratio > 1.0 - 1e-6 ? 1.0 - 1e-6 : ratio);
+                    o[5] = (float)log(ratio / (1.0 - ratio));
+                }
+            }
+            break;
+        }
+        if (r.fallback) break;
+        const double e = exp(lk + z), res = fabs(z + 0.5 * e * (1.0 - exp(-2.0 * z)) - S);
+        if (ok && !(res > 1e-10 * (1.0 + S))) break;
+        r.fallback = true;
+        z = S;
+        cap = maxit;
+    }
     const double V = 2.0 * V0 * exp(-psi / a + z) * 0.5 * (1.0 - exp(-2.0 * z));
     r.V = tq < 0.0 ? -V : V;
     return r;
 }
 
-__device__ inline void write_x(const VArgs &A, int64_t i, double d1, double d2)
+// Component c of the deficit, in both layouts.
+__device__ inline void write_xc(const VArgs &A, int64_t i, int c, double d)
 {
     const int64_t P = ((A.n + 16 + 7) / 8) * 8;
     if (A.x_fp32) {
         float *x = (float *)A.x;
-        x[2 * i] = (float)d1; x[2 * i + 1] = (float)d2; x[2 * P + i] = (float)d1; x[3 * P + i] = (float)d2;
+        x[2 * i + c] = x[(2 + c) * P + i] = (float)d;
     } else {
         double *x = (double *)A.x;
-        x[2 * i] = d1; x[2 * i + 1] = d2; x[2 * P + i] = d1; x[3 * P + i] = d2;
+        x[2 * i + c] = x[(2 + c) * P + i] = d;
     }
 }
 
+__device__ inline void write_x(const VArgs &A, int64_t i, double d1, double d2)
+{
+    write_xc(A, i, 0, d1);
+    write_xc(A, i, 1, d2);
+}
+
+// Two lanes an element, one traction component each: the stage is a chain of some ten FP64
+// transcendentals per component, and with both in one thread (and a copy of the solve for each)
+// it took 11.5 us for 9,000 elements on 71 CTAs, @@ now.  The Newton counters go up once per
+// CTA; one atomic per warp and counter queued on the same words.
 __global__ void __launch_bounds__(VM_THREADS) k_vmode_stage(VArgs A, int s)
 {
     __shared__ double red[VM_THREADS / 32][2];
+    __shared__ unsigned cnt[VM_THREADS / 32][4];
     __shared__ int s_last;
     // MLP parameters are read in place through the read-only cache: only solves that
     // fail the undamped-start test touch them, and a warp's lanes read the same weight.
     const bool use_mlp = (A.seed_mode == 2 || A.seed_mode == 3) && A.mlp;
     const float *__restrict__ P = A.mlp;
     const int n = A.n;
+    const int c = threadIdx.x & 1;
+    const int64_t i = (int64_t)blockIdx.x * (VM_THREADS / 2) + (threadIdx.x >> 1);
+    const bool on = i < n;
+    asm volatile("griddepcontrol.wait;" ::: "memory");    // launched while the row reduction ends (12 stages: 16 us)
     const double h = A.ctrl[0], t0 = A.ctrl[2];
     const double ts = t0 + kC[s - 1] * h;
     double Emax = 0.0;
-    unsigned long long its = 0, solves = 0, itmax = 0, fb = 0;
-    const int64_t i = (int64_t)blockIdx.x * VM_THREADS + threadIdx.x;
-    if (i < n) {
-        double *k = A.k;
+    Solve r{0.0, 0, false};
+    double *k = A.k;
+    double psi = 0.0;
+    if (on) {
         // stage state
-        double ys[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            double acc = 0.0;
-            for (int j = 0; j < s - 1; ++j) acc += kA[s - 1][j] * k[((int64_t)j * 3 + c) * n + i];
-            ys[c] = A.y0[(int64_t)c * n + i] + h * acc;
-        }
-        const double a = A.a[i], b = A.b[i];
-        const double tq1 = A.tq1[i] - A.mv[3 * i] + A.shear_loading[i] * ts;
-        const double tq2 = A.tq2[i] - A.mv[3 * i + 1] + A.shear_loading[i] * ts;
+        double acc = 0.0;
+        for (int j = 0; j < s - 1; ++j) acc += kA[s - 1][j] * k[((int64_t)j * 3 + 2) * n + i];
+        psi = A.y0[(int64_t)2 * n + i] + h * acc;
+        const double tq = (c ? A.tq2 : A.tq1)[i] - A.mv[3 * i + c] + A.shear_loading[i] * ts;
         const double sig = A.sig0[i] + A.mv[3 * i + 2] + A.normal_loading[i] * ts;
-        const Solve r1 = vsolve(tq1, sig, ys[2], a, b, A.V0, A.eta, A.V[i], A.seed_mode, use_mlp ? P : nullptr,
-                                A.mlp_gate, A.newton_tol, A.newton_max, A.log_x, A.log_n, A.log_cap);
-        const Solve r2 = vsolve(tq2, sig, ys[2], a, b, A.V0, A.eta, A.V[n + i], A.seed_mode, use_mlp ? P : nullptr,
-                                A.mlp_gate, A.newton_tol, A.newton_max, A.log_x, A.log_n, A.log_cap);
-        A.V[i] = r1.V;
-        A.V[n + i] = r2.V;
-        its = r1.iters + r2.iters;
-        solves = 2;
-        itmax = r1.iters > r2.iters ? r1.iters : r2.iters;
-        fb = (r1.fallback ? 1 : 0) + (r2.fallback ? 1 : 0);
-        const double Vm = sqrt(r1.V * r1.V + r2.V * r2.V);
-        double arg = (A.f0[i] - ys[2]) / b;
+        r = vsolve(tq, sig, psi, A.a[i], A.b[i], A.V0, A.eta, A.V[(int64_t)c * n + i], A.seed_mode, use_mlp ? P : nullptr,
+                   A.mlp_gate, A.newton_tol, A.newton_max, A.log_x, A.log_n, A.log_cap);
+    }
+    const double Vo = __shfl_xor_sync(0xffffffffu, r.V, 1);
+    if (on) {
+        A.V[(int64_t)c * n + i] = r.V;
+        const double V1 = c ? Vo : r.V, V2 = c ? r.V : Vo;
+        const double Vm = sqrt(V1 * V1 + V2 * V2);
+        const double b = A.b[i];
+        double arg = (A.f0[i] - psi) / b;
         arg = arg > 700.0 ? 700.0 : (arg < -700.0 ? -700.0 : arg);
         const double dpsi = b / A.dc[i] * (A.V0 * exp(arg) - Vm);
-        k[((int64_t)(s - 1) * 3 + 0) * n + i] = r1.V;
-        k[((int64_t)(s - 1) * 3 + 1) * n + i] = r2.V;
-        k[((int64_t)(s - 1) * 3 + 2) * n + i] = dpsi;
+        k[((int64_t)(s - 1) * 3 + c) * n + i] = r.V;
+        if (c == 0) k[((int64_t)(s - 1) * 3 + 2) * n + i] = dpsi;
+        // sum over the stages up to this one of the tableau row's weights times k, component q
+        auto combine = [&](const double *w, int q) {
+            double acc = 0.0;
+            for (int j = 0; j < s - 1; ++j) acc += w[j] * k[((int64_t)j * 3 + q) * n + i];
+            return acc + w[s - 1] * (q == 2 ? dpsi : r.V);
+        };
         if (s < 7) {
             // next stage state and its deficit for the next matvec
-            double yn[3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                double acc = 0.0;
-                for (int j = 0; j < s; ++j) acc += kA[s][j] * k[((int64_t)j * 3 + c) * n + i];
-                yn[c] = A.y0[(int64_t)c * n + i] + h * acc;
+            const double yn = A.y0[(int64_t)c * n + i] + h * combine(kA[s], c);
+            if (s == 6) {
+                A.y5[(int64_t)c * n + i] = yn;
+                if (c == 0) A.y5[(int64_t)2 * n + i] = A.y0[(int64_t)2 * n + i] + h * combine(kA[s], 2);
             }
-            if (s == 6)
-#pragma unroll
-                for (int c = 0; c < 3; ++c) A.y5[(int64_t)c * n + i] = yn[c];
             const double tn = t0 + kC[s] * h;
-            write_x(A, i, yn[0] - A.vplc[i] * A.cr0[i] * tn, yn[1] - A.vplc[i] * A.sr0[i] * tn);
+            write_xc(A, i, c, yn - A.vplc[i] * (c ? A.sr0 : A.cr0)[i] * tn);
         } else {
-            double e[3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                double acc = 0.0;
-                for (int j = 0; j < 7; ++j) acc += kB4[j] * k[((int64_t)j * 3 + c) * n + i];
-                const double y4 = A.y0[(int64_t)c * n + i] + h * acc;
-                e[c] = fabs(A.y5[(int64_t)c * n + i] - y4);
-            }
-            const double y51 = A.y5[i], y52 = A.y5[n + i], y5p = A.y5[2 * (int64_t)n + i];
-            Emax = fmax(fmax(e[2] / fabs(y5p), e[0] / (fabs(y51) + A.atol)), e[1] / (fabs(y52) + A.atol));
-            if (Emax != Emax) Emax = INFINITY;
+            const double yc = A.y5[(int64_t)c * n + i], yp = A.y5[(int64_t)2 * n + i];
+            const double ec = fabs(yc - (A.y0[(int64_t)c * n + i] + h * combine(kB4, c)));
+            const double ep = fabs(yp - (A.y0[(int64_t)2 * n + i] + h * combine(kB4, 2)));
+            Emax = fmax(ep / fabs(yp), ec / (fabs(yc) + A.atol));
         }
     }
+    // both components' terms; infinite when all three are NaN
+    Emax = fmax(Emax, __shfl_xor_sync(0xffffffffu, Emax, 1));
+    if (Emax != Emax) Emax = INFINITY;
     // Newton statistics
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        its += __shfl_down_sync(0xffffffffu, its, o);
-        solves += __shfl_down_sync(0xffffffffu, solves, o);
-        fb += __shfl_down_sync(0xffffffffu, fb, o);
-        const unsigned long long om = __shfl_down_sync(0xffffffffu, itmax, o);
-        itmax = om > itmax ? om : itmax;
+    unsigned its = on ? r.iters : 0, solves = on, itmax = its, fb = r.fallback;
+    its = __reduce_add_sync(0xffffffffu, its);
+    solves = __reduce_add_sync(0xffffffffu, solves);
+    itmax = __reduce_max_sync(0xffffffffu, itmax);
+    fb = __reduce_add_sync(0xffffffffu, fb);
+    if ((threadIdx.x & 31) == 0) {
+        unsigned *o = cnt[threadIdx.x >> 5];
+        o[0] = its; o[1] = solves; o[2] = itmax; o[3] = fb;
     }
-    if ((threadIdx.x & 31) == 0 && solves) {
-        atomicAdd(A.stats, its);
-        atomicAdd(A.stats + 1, solves);
-        atomicMax(A.stats + 2, itmax);
-        if (fb) atomicAdd(A.stats + 3, fb);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < VM_THREADS / 32; ++w) {
+            its += cnt[w][0];
+            solves += cnt[w][1];
+            itmax = cnt[w][2] > itmax ? cnt[w][2] : itmax;
+            fb += cnt[w][3];
+        }
+        atomicAdd(A.stats, (unsigned long long)its);
+        atomicAdd(A.stats + 1, (unsigned long long)solves);
+        atomicMax(A.stats + 2, (unsigned long long)itmax);
+        if (fb) atomicAdd(A.stats + 3, (unsigned long long)fb);
     }
     if (s < 7) return;
     // stage 7: grid max of the error ratio; the last CTA decides (accept / reject)
@@ -406,6 +394,9 @@ __global__ void k_vmode_deficit(VArgs A)
 
 PQ3D_EXPORT size_t pq3d_vmode_args_bytes(void) { return sizeof(VArgs); }
 
+// CTAs of a stage (two threads an element): doubles of VArgs.blk.
+PQ3D_EXPORT int pq3d_vmode_grid(int n) { return (n + VM_THREADS / 2 - 1) / (VM_THREADS / 2); }
+
 // stage 1..7 of the current attempt (stage 1 only at start-up, after a matvec of the
 // step-start deficit); -1: write the step-start deficit; 0: finalize the attempt.
 PQ3D_EXPORT int pq3d_vmode_stage(const void *args, int stage, cudaStream_t stream)
@@ -420,9 +411,16 @@ PQ3D_EXPORT int pq3d_vmode_stage(const void *args, int stage, cudaStream_t strea
         k_vmode_finalize<<<grid, VM_THREADS, 0, stream>>>(A);
     } else {
         if (!A.mv || !A.y5 || !A.blk || !A.bar || !A.stats) return PQ3D_ERR_ARG;
-        k_vmode_stage<<<grid, VM_THREADS, 0, stream>>>(A, stage);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)pq3d_vmode_grid(A.n));
+        cfg.blockDim = dim3(VM_THREADS);
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        PQ3D_CHECK(cudaLaunchKernelEx(&cfg, k_vmode_stage, A, stage));
     }
     return pq3d_launch_status();
 }
-
-PQ3D_EXPORT int pq3d_vmode_grid(int n) { return (n + VM_THREADS - 1) / VM_THREADS; }
