@@ -22,7 +22,7 @@
 //               slot rows = U_c t_c.  Launched with programmatic stream
 //               serialization, so its dense items run in k_dense_v's tail; the
 //               U tasks wait for k_dense_v.
-//   k_u         (FP64) the U tasks as a plain launch after k_dense_v.
+//   k_u         (FP64) the U tasks, likewise behind k_dense_v.
 //   k_rowsum    y[i] = sum of row i's slots (FP64), plus optional loading terms
 //               (skipped when the step kernel sums the slots itself)
 #include <algorithm>

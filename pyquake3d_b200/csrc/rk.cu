@@ -56,6 +56,13 @@ __device__ __forceinline__ unsigned atom_add_acq_rel_u32(unsigned *p, unsigned x
     return old;
 }
 
+__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long k)
+{
+    const unsigned hi = (unsigned)(k >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)k : 0u);
+    return ((unsigned long long)mh << 32) | ml;
+}
+
 // Grid-wide NaN-propagating max of four values that are >= 0 or +NaN, in one
 // phase.  Every CTA folds its block maximum into a result slot with 64-bit
 // atomicMax on the bit patterns (for such values the unsigned order of the
@@ -71,31 +78,30 @@ __device__ __forceinline__ unsigned atom_add_acq_rel_u32(unsigned *p, unsigned x
 template <int NT>
 __device__ bool grid_max4(double *v, unsigned long long *slots3, unsigned *bar, int attempt, double *ctrl)
 {
-    __shared__ double wred[NT / 32][4];
+    static_assert(NT == 256, "eight warps: lane 8 q + w reduces maximum q of warp w");
+    __shared__ unsigned long long wred[4][NT / 32];
     __shared__ double s_res[4];
     __shared__ int s_ok;
+    const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
-#pragma unroll 1
-        for (int o = 16; o > 0; o >>= 1) v[q] = nanmax(v[q], __shfl_down_sync(0xffffffffu, v[q], o));
-    if ((threadIdx.x & 31) == 0)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) wred[threadIdx.x >> 5][q] = v[q];
+    for (int q = 0; q < 4; ++q) {
+        const unsigned long long m = warp_max_u64((unsigned long long)__double_as_longlong(v[q]));
+        if (lane == 0) wred[q][threadIdx.x >> 5] = m;
+    }
     __syncthreads();
     if (threadIdx.x < 32) {
-        // lanes 0..3: one maximum each
         unsigned long long *r = slots3 + 4 * (attempt % 3);
-        const int q = threadIdx.x;
-        if (q < 4) {
-            double w = wred[0][q];
-            for (int k = 1; k < NT / 32; ++k) w = nanmax(w, wred[k][q]);
-            atomicMax(r + q, (unsigned long long)__double_as_longlong(w));
+        unsigned long long m = wred[lane >> 3][lane & 7];
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) {
+            const unsigned long long x = __shfl_xor_sync(0xffffffffu, m, o);
+            m = x > m ? x : m;
         }
+        if ((lane & 7) == 0) atomicMax(r + (lane >> 3), m);
         __syncwarp();
-        if (q == 0) {
+        if (lane == 0) {
             const unsigned target = (unsigned)(attempt + 1) * gridDim.x;
             int ok = 1;
-            __threadfence();
             if (atom_add_acq_rel_u32(bar, 1u) + 1u == target) {
                 unsigned long long *z = slots3 + 4 * ((attempt + 2) % 3);
                 for (int e = 0; e < 4; ++e) __stcg(z + e, 0ull);
@@ -113,7 +119,7 @@ __device__ bool grid_max4(double *v, unsigned long long *slots3, unsigned *bar, 
             s_ok = ok;
         }
         __syncwarp();
-        if (q < 4) s_res[q] = __longlong_as_double((long long)__ldcg(r + q));
+        if (lane < 4) s_res[lane] = __longlong_as_double((long long)__ldcg(r + lane));
     }
     __syncthreads();
 #pragma unroll
@@ -126,10 +132,10 @@ __device__ bool grid_max4(double *v, unsigned long long *slots3, unsigned *bar, 
 #endif
 // Two 256-thread CTAs per SM, R rows per CTA (rs_rows): at 60k elements one element per thread,
 // below that as few rows per CTA as fill the grid, so that all SMs share the latency-bound
-// element work and every thread the row sums.  B200, us per launch, against 256 rows per CTA:
-// 1,936 elements 47 -> 21, 9,000 33 -> 21, 20,480 24 -> 23, 60k 43 -> 38.  Cycles of a launch at
-// 20,480 (clock64 stamps): row sums 8,300, stages 14,900, grid maximum 7,900, accept 4,400,
-// end of step 5,300.
+// element work and every thread the row sums.  B200, us per launch, against 256 rows per CTA and
+// unrolled stages: 1,936 elements 43.5 -> 19.0, 5,000 22.5 -> 17.7, 20,480 24.0 -> 22.5, 60k 42.9 -> 35.6.
+// Cycles of a launch at 20,480 (clock64 stamps): row sums 9,600, stages 14,200 (seven derivatives
+// of 930, their combinations 430 each), grid maximum 6,300, accept 5,400, end of step 3,000.
 #ifndef PQ3D_RK_MINB
 #define PQ3D_RK_MINB 2
 #endif
@@ -171,6 +177,10 @@ __global__ void __launch_bounds__(RK_THREADS, PQ3D_RK_MINB) k_rk_step(RkArgs A)
         if (controller_decide(c, E, A.reltol, forced)) break;
     }
     const double h = c.h;
+    // the size after this step: two powers, by a thread of the last warp (idle when R <= 224)
+    // while the others update the state
+    __shared__ double s_next;
+    if (threadIdx.x == RK_THREADS - 1 && c.accepted) s_next = controller_next(h, E, A.reltol);
     const bool accepted = c.accepted;
     const int nrjct = c.nrjct, attempt = c.attempt;
 
@@ -184,32 +194,39 @@ __global__ void __launch_bounds__(RK_THREADS, PQ3D_RK_MINB) k_rk_step(RkArgs A)
             mv2 = fmax(mv2, fabs(v2));
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        mv1 = fmax(mv1, __shfl_down_sync(0xffffffffu, mv1, o));
-        mv2 = fmax(mv2, __shfl_down_sync(0xffffffffu, mv2, o));
+    __shared__ unsigned long long vred[2][RK_THREADS / 32];
+    {
+        // >= 0 and never NaN: ordered bits
+        const unsigned long long m1 = warp_max_u64((unsigned long long)__double_as_longlong(mv1)),
+                                 m2 = warp_max_u64((unsigned long long)__double_as_longlong(mv2));
+        if ((threadIdx.x & 31) == 0) {
+            vred[0][threadIdx.x >> 5] = m1;
+            vred[1][threadIdx.x >> 5] = m2;
+        }
     }
-    __shared__ double vred[RK_THREADS / 32][2];
-    if ((threadIdx.x & 31) == 0) { vred[threadIdx.x >> 5][0] = mv1; vred[threadIdx.x >> 5][1] = mv2; }
     __syncthreads();
     // every CTA folds its slip-rate maxima (>= 0, never NaN) into two words; the last one to
     // finish the step updates ctrl, read ahead of its arrival
     if (threadIdx.x == 0) {
-        double w1 = vred[0][0], w2 = vred[0][1];
-        for (int k = 1; k < RK_THREADS / 32; ++k) { w1 = fmax(w1, vred[k][0]); w2 = fmax(w2, vred[k][1]); }
+        unsigned long long u1 = vred[0][0], u2 = vred[1][0];
+#pragma unroll
+        for (int k = 1; k < RK_THREADS / 32; ++k) {
+            u1 = vred[0][k] > u1 ? vred[0][k] : u1;
+            u2 = vred[1][k] > u2 ? vred[1][k] : u2;
+        }
         const double c2 = A.ctrl[2], c4 = A.ctrl[4], c8 = A.ctrl[8], c9 = A.ctrl[9], c10 = A.ctrl[10];
-        atomicMax(slots3 + 12, (unsigned long long)__double_as_longlong(w1));
-        atomicMax(slots3 + 13, (unsigned long long)__double_as_longlong(w2));
+        atomicMax(slots3 + 12, u1);
+        atomicMax(slots3 + 13, u2);
         __threadfence();
         if (atomicAdd(A.bar + 2, 1u) != gridDim.x - 1) return;
         __threadfence();
-        w1 = __longlong_as_double((long long)__ldcg(slots3 + 12));
-        w2 = __longlong_as_double((long long)__ldcg(slots3 + 13));
+        const double w1 = __longlong_as_double((long long)__ldcg(slots3 + 12));
+        const double w2 = __longlong_as_double((long long)__ldcg(slots3 + 13));
         A.bar[2] = 0u;
         A.bar[0] = 0u;
         for (int q = 0; q < 14; ++q) slots3[q] = 0ull;
         if (accepted) {
-            const double t = c2 + h, dtnext = controller_next(h, E, A.reltol);
+            const double t = c2 + h, dtnext = s_next;
             A.ctrl[2] = t;
             A.ctrl[0] = dtnext;   // next dttry
             A.ctrl[1] = h;        // accepted step
