@@ -233,7 +233,9 @@ int pq3d_rk_rows_finish(double *d_pc, const double *d_V8, cudaStream_t stream);
  * controller.  Rows of a fault are a contiguous tree-order range; CTA tasks of
  * at most pq3d_ens_task_rows() rows never span two faults.  ctrl holds 16
  * doubles per fault (layout of the pq3d_rk_step control block), hist 6 doubles
- * per (step, fault). */
+ * per (step, fault), fstate 24 doubles per fault, zeroed once.  With as many
+ * CTAs as tasks each fault steps on its own; with fewer the faults advance in
+ * lock-step attempts. */
 size_t pq3d_ens_args_bytes(void);
 int pq3d_ens_task_rows(void);
 int pq3d_ens_grid(int n_tasks);

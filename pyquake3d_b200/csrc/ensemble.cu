@@ -6,14 +6,15 @@
 // The step kernel does, per fault, exactly what k_rk_step does for one fault
 // (the reference's simu_forward after the load, src/QDsim.py:892-996): DP5(4)
 // attempts with the frozen load, NaN-propagating error maxima over the fault's
-// elements, the reference controller, and the accepted-step update.  Faults
-// advance in lock-step attempts: a fault whose step is accepted (or given up)
-// is skipped by the later attempts of the others.
+// elements, the reference controller, and the accepted-step update.  With a CTA per task
+// (k_rk_faults) each fault runs on its own; with several tasks per CTA (k_rk_ensemble) faults
+// advance in lock-step attempts, and one whose step is accepted (or given up) is skipped by
+// the later attempts of the others.
 //
 // Work is split into CTA tasks of at most ENS_THREADS rows of one fault; the
 // fused row sums of a task's rows are done by its CTA before its first attempt
-// (staged slot lists, rowsum_cta).  After
-// each attempt the last CTA to arrive reduces the per-task maxima of every
+// (staged slot lists, rowsum_cta).  In lock step,
+// after each attempt the last CTA to arrive reduces the per-task maxima of every
 // running fault, applies the controller, publishes the per-fault state and
 // releases the others (bounded spins; PQ3D_ERR_TIMEOUT in every fault's status).
 #include "pq3d_common.cuh"
@@ -24,7 +25,8 @@ using namespace pq3d_rk;
 
 constexpr int ENS_THREADS = 256;
 constexpr int ENS_CTRL = 16;    // doubles of per-fault control (layout of the single-fault ctrl)
-constexpr int ENS_FSTATE = 8;   // doubles of per-fault attempt state
+constexpr int ENS_FSTATE = 24;  // doubles of per-fault scratch: attempt state of the lock-step kernel, and
+constexpr int ENS_WORDS = 8;    // from here on the 14 + 1 words a fault's CTAs meet at
 constexpr int ENS_MAX_ATTEMPTS = 64;
 
 struct EnsArgs {
@@ -41,7 +43,8 @@ struct EnsArgs {
     const int32_t *fault_task; // tasks of fault s: [fault_task[s], fault_task[s+1])
     double *tmax;              // 4 doubles per task
     double *ctrl;              // ENS_CTRL doubles per fault
-    double *fstate;            // ENS_FSTATE doubles per fault: h, dtnext, nrjct, attempt, phase
+    double *fstate;            // ENS_FSTATE doubles per fault: h, dtnext, nrjct, attempt, phase; meeting
+                               // words at ENS_WORDS (zeroed once)
     double *hist;              // 6 doubles per (step, fault), may be null
     const double *hforce;      // dt replay: step s of fault f takes hforce[s * n_faults + f]
     unsigned *bar;             // [0] arrivals, [1] generation, [2] end-of-step count, [3] all-done flag
@@ -276,6 +279,36 @@ __global__ void __launch_bounds__(ENS_THREADS) k_rk_ensemble(EnsArgs A)
     }
 }
 
+struct OneFault {
+    const EnsArgs &A;
+    int s;
+    __device__ double *ctrl() const { return A.ctrl + (int64_t)ENS_CTRL * s; }
+    __device__ double *hist() const { return A.hist ? A.hist + 6 * ((int64_t)A.step_index * A.n_faults + s) : nullptr; }
+    __device__ double *ctrl_host() const { return nullptr; }
+    __device__ unsigned long long *slots3() const
+    {
+        return (unsigned long long *)(A.fstate + (int64_t)ENS_FSTATE * s + ENS_WORDS);
+    }
+    __device__ unsigned *bar() const { return (unsigned *)(slots3() + 14); }
+    __device__ unsigned *end() const { return bar() + 1; }
+    __device__ unsigned parties() const { return (unsigned)(A.fault_task[s + 1] - A.fault_task[s]); }
+};
+
+// One CTA per task: a fault's CTAs meet only one another, as k_rk_step's do, so no fault waits for
+// another's attempts, the maxima are folded in one phase and the next size is computed beside the
+// state update.  B200, six faults, 12.6k elements: 18.9 us a launch, 28.1 in lock step.
+template <typename TA>
+__global__ void __launch_bounds__(ENS_THREADS, 2) k_rk_faults(EnsArgs A)
+{
+    const int t = blockIdx.x, s = A.task_fault[t];
+    const int64_t r0 = A.task_row[t], r1 = A.task_row[t + 1];
+    if (A.fuse_rowsum) rowsum_cta<ENS_THREADS, TA>(A, r0, r1, (int)(r1 - r0 + 15) & ~15);
+    const bool forced = A.hforce != nullptr;
+    const double h = forced ? A.hforce[(int64_t)A.step_index * A.n_faults + s] : A.ctrl[(int64_t)ENS_CTRL * s];
+    const StepCtl c{h, 0.0, 0, 0, false};
+    step_fault<ENS_THREADS>(A, OneFault{A, s}, c, forced, r0 + threadIdx.x, r1, ENS_THREADS);
+}
+
 }  // namespace
 
 PQ3D_EXPORT size_t pq3d_ens_args_bytes(void) { return sizeof(EnsArgs); }
@@ -287,10 +320,13 @@ PQ3D_EXPORT int pq3d_ens_grid(int n_tasks)
     if (n_tasks <= 0) return -1;
     if (cudaGetDevice(&dev) != cudaSuccess) return -1;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -1;
-    int per32 = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_rk_ensemble<double>, ENS_THREADS, 0) != cudaSuccess) return -1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per32, k_rk_ensemble<float>, ENS_THREADS, 0) != cudaSuccess) return -1;
-    per = per32 < per ? per32 : per;
+    const void *kernels[] = {(const void *)k_rk_faults<double>, (const void *)k_rk_faults<float>,
+                             (const void *)k_rk_ensemble<double>, (const void *)k_rk_ensemble<float>};
+    for (const void *k : kernels) {
+        int p = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, k, ENS_THREADS, 0) != cudaSuccess) return -1;
+        if (k == kernels[0] || p < per) per = p;
+    }
     const int cap = sms * per;
     return n_tasks < cap ? n_tasks : cap;
 }
@@ -316,6 +352,11 @@ PQ3D_EXPORT int pq3d_ens_step(const void *args, int grid, cudaStream_t stream)
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    PQ3D_CHECK(cudaLaunchKernelEx(&cfg, A.slots_fp32 ? k_rk_ensemble<float> : k_rk_ensemble<double>, A));
+    // a CTA per task needs every task co-resident; above that (75k rows at 256 a task, or more
+    // faults than CTAs) the CTAs take several tasks each, in lock step
+    if (grid == A.n_tasks)
+        PQ3D_CHECK(cudaLaunchKernelEx(&cfg, A.slots_fp32 ? k_rk_faults<float> : k_rk_faults<double>, A));
+    else
+        PQ3D_CHECK(cudaLaunchKernelEx(&cfg, A.slots_fp32 ? k_rk_ensemble<float> : k_rk_ensemble<double>, A));
     return PQ3D_OK;
 }

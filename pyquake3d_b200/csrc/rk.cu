@@ -42,91 +42,6 @@ struct RkArgs {
     double h_in;         // > 0: the step's trial size (instead of ctrl[0])
 };
 
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p)
-{
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ unsigned atom_add_acq_rel_u32(unsigned *p, unsigned x)
-{
-    unsigned old;
-    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(x) : "memory");
-    return old;
-}
-
-__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long k)
-{
-    const unsigned hi = (unsigned)(k >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
-    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)k : 0u);
-    return ((unsigned long long)mh << 32) | ml;
-}
-
-// Grid-wide NaN-propagating max of four values that are >= 0 or +NaN, in one
-// phase.  Every CTA folds its block maximum into a result slot with 64-bit
-// atomicMax on the bit patterns (for such values the unsigned order of the
-// bits is the order of the values, and +NaN lies above +inf, so the fold is
-// nanmax), then arrives on bar[0] with acquire-release semantics; a CTA goes on
-// once bar[0] reaches (attempt + 1) * gridDim.x and reads the slot.  Attempts
-// rotate over three slots of four: the CTA that arrives last at attempt a
-// clears slot (a + 2) % 3, which every CTA finished reading before it arrived
-// at a and which no CTA touches before the next barrier.  The last CTA to
-// finish the step clears bar[0] and the slots.  All CTAs return the same four
-// values.  Bounded spin: on timeout ctrl[4] = PQ3D_ERR_TIMEOUT and false is
-// returned.
-template <int NT>
-__device__ bool grid_max4(double *v, unsigned long long *slots3, unsigned *bar, int attempt, double *ctrl)
-{
-    static_assert(NT == 256, "eight warps: lane 8 q + w reduces maximum q of warp w");
-    __shared__ unsigned long long wred[4][NT / 32];
-    __shared__ double s_res[4];
-    __shared__ int s_ok;
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const unsigned long long m = warp_max_u64((unsigned long long)__double_as_longlong(v[q]));
-        if (lane == 0) wred[q][threadIdx.x >> 5] = m;
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        unsigned long long *r = slots3 + 4 * (attempt % 3);
-        unsigned long long m = wred[lane >> 3][lane & 7];
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1) {
-            const unsigned long long x = __shfl_xor_sync(0xffffffffu, m, o);
-            m = x > m ? x : m;
-        }
-        if ((lane & 7) == 0) atomicMax(r + (lane >> 3), m);
-        __syncwarp();
-        if (lane == 0) {
-            const unsigned target = (unsigned)(attempt + 1) * gridDim.x;
-            int ok = 1;
-            if (atom_add_acq_rel_u32(bar, 1u) + 1u == target) {
-                unsigned long long *z = slots3 + 4 * ((attempt + 2) % 3);
-                for (int e = 0; e < 4; ++e) __stcg(z + e, 0ull);
-            } else {
-                long long it = 0;
-                while (ld_acquire_u32(bar) < target) {
-                    if (++it > (1LL << 24)) {
-                        ctrl[4] = (double)PQ3D_ERR_TIMEOUT;
-                        ok = 0;
-                        break;
-                    }
-                    __nanosleep(32);
-                }
-            }
-            s_ok = ok;
-        }
-        __syncwarp();
-        if (lane < 4) s_res[lane] = __longlong_as_double((long long)__ldcg(r + lane));
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 4; ++q) v[q] = s_res[q];
-    return s_ok != 0;
-}
-
 #ifndef PQ3D_RK_THREADS
 #define PQ3D_RK_THREADS 256
 #endif
@@ -140,6 +55,17 @@ __device__ bool grid_max4(double *v, unsigned long long *slots3, unsigned *bar, 
 #define PQ3D_RK_MINB 2
 #endif
 constexpr int RK_THREADS = PQ3D_RK_THREADS;   // CTA size of the step kernel
+
+struct WholeGrid {
+    const RkArgs &A;
+    __device__ double *ctrl() const { return A.ctrl; }
+    __device__ double *hist() const { return A.hist ? A.hist + 6 * (int64_t)A.step_index : nullptr; }
+    __device__ double *ctrl_host() const { return A.ctrl_host; }
+    __device__ unsigned long long *slots3() const { return (unsigned long long *)(A.blk + 10 * (int64_t)gridDim.x); }
+    __device__ unsigned *bar() const { return A.bar; }
+    __device__ unsigned *end() const { return A.bar + 2; }
+    __device__ unsigned parties() const { return gridDim.x; }
+};
 
 // TA: type of the matvec's slots (a kernel each, for half the code).
 template <typename TA>
@@ -155,103 +81,9 @@ __global__ void __launch_bounds__(RK_THREADS, PQ3D_RK_MINB) k_rk_step(RkArgs A)
         for (int64_t base = (int64_t)blockIdx.x * R; base < n; base += stride)
             rowsum_cta<RK_THREADS, TA>(A, base, n, R);
     }
-    unsigned long long *slots3 = (unsigned long long *)(A.blk + 10 * (int64_t)gridDim.x);
     const bool forced = A.hforce != nullptr;
-    StepCtl c{forced ? A.hforce[A.step_index] : (A.h_in > 0.0 ? A.h_in : A.ctrl[0]), 0.0, 0, 0, false};
-    c.dtnext = c.h;
-    double E[4];
-
-    while (true) {
-        double m1 = 0.0, g1 = 0.0, g2 = 0.0, g3 = 0.0;  // max relative errors, NaN-propagating
-        for (int64_t i = tid0; i < n; i += stride) {
-            double e[4];
-            dp54_element(A, i, c.h, e);
-            m1 = nanmax(m1, e[0]);
-            g1 = nanmax(g1, e[1]);
-            g2 = nanmax(g2, e[2]);
-            g3 = nanmax(g3, e[3]);
-        }
-        // grid-wide maxima of (m1, g1, g2, g3); identical in every CTA
-        E[0] = m1; E[1] = g1; E[2] = g2; E[3] = g3;
-        if (!grid_max4<RK_THREADS>(E, slots3, A.bar, c.attempt, A.ctrl)) return;
-        if (controller_decide(c, E, A.reltol, forced)) break;
-    }
-    const double h = c.h;
-    // the size after this step: two powers, by a thread of the last warp (idle when R <= 224)
-    // while the others update the state
-    __shared__ double s_next;
-    if (threadIdx.x == RK_THREADS - 1 && c.accepted) s_next = controller_next(h, E, A.reltol);
-    const bool accepted = c.accepted;
-    const int nrjct = c.nrjct, attempt = c.attempt;
-
-    // accepted step: state update (src/QDsim.py:960-993) and next deficit (:902-903)
-    double mv1 = 0.0, mv2 = 0.0;
-    if (accepted) {
-        for (int64_t i = tid0; i < n; i += stride) {
-            double v1, v2;
-            accept_element(A, i, h, v1, v2);
-            mv1 = fmax(mv1, fabs(v1));
-            mv2 = fmax(mv2, fabs(v2));
-        }
-    }
-    __shared__ unsigned long long vred[2][RK_THREADS / 32];
-    {
-        // >= 0 and never NaN: ordered bits
-        const unsigned long long m1 = warp_max_u64((unsigned long long)__double_as_longlong(mv1)),
-                                 m2 = warp_max_u64((unsigned long long)__double_as_longlong(mv2));
-        if ((threadIdx.x & 31) == 0) {
-            vred[0][threadIdx.x >> 5] = m1;
-            vred[1][threadIdx.x >> 5] = m2;
-        }
-    }
-    __syncthreads();
-    // every CTA folds its slip-rate maxima (>= 0, never NaN) into two words; the last one to
-    // finish the step updates ctrl, read ahead of its arrival
-    if (threadIdx.x == 0) {
-        unsigned long long u1 = vred[0][0], u2 = vred[1][0];
-#pragma unroll
-        for (int k = 1; k < RK_THREADS / 32; ++k) {
-            u1 = vred[0][k] > u1 ? vred[0][k] : u1;
-            u2 = vred[1][k] > u2 ? vred[1][k] : u2;
-        }
-        const double c2 = A.ctrl[2], c4 = A.ctrl[4], c8 = A.ctrl[8], c9 = A.ctrl[9], c10 = A.ctrl[10];
-        atomicMax(slots3 + 12, u1);
-        atomicMax(slots3 + 13, u2);
-        __threadfence();
-        if (atomicAdd(A.bar + 2, 1u) != gridDim.x - 1) return;
-        __threadfence();
-        const double w1 = __longlong_as_double((long long)__ldcg(slots3 + 12));
-        const double w2 = __longlong_as_double((long long)__ldcg(slots3 + 13));
-        A.bar[2] = 0u;
-        A.bar[0] = 0u;
-        for (int q = 0; q < 14; ++q) slots3[q] = 0ull;
-        if (accepted) {
-            const double t = c2 + h, dtnext = s_next;
-            A.ctrl[2] = t;
-            A.ctrl[0] = dtnext;   // next dttry
-            A.ctrl[1] = h;        // accepted step
-            A.ctrl[3] = nrjct;
-            A.ctrl[5] = w1;
-            A.ctrl[6] = w2;
-            A.ctrl[8] = c8 + 1.0;
-            A.ctrl[9] = c9 + nrjct;
-            A.ctrl[10] = c10 + attempt;
-            if (A.hist) {
-                double *hh = A.hist + 6 * (int64_t)A.step_index;
-                hh[0] = h; hh[1] = dtnext; hh[2] = t; hh[3] = w1; hh[4] = w2; hh[5] = nrjct;
-            }
-        } else {
-            A.ctrl[1] = h;
-            A.ctrl[3] = nrjct;
-            if (c4 == 0.0) A.ctrl[4] = (double)PQ3D_ERR_DT;
-        }
-        if (A.ctrl_host) {
-            // the host's copy, sequence number last (a step that ended early leaves it stale)
-            for (int k = 0; k < 11; ++k) A.ctrl_host[k] = A.ctrl[k];
-            __threadfence_system();
-            A.ctrl_host[15] = (double)A.step_index + 1.0;
-        }
-    }
+    const StepCtl c{forced ? A.hforce[A.step_index] : (A.h_in > 0.0 ? A.h_in : A.ctrl[0]), 0.0, 0, 0, false};
+    step_fault<RK_THREADS>(A, WholeGrid{A}, c, forced, tid0, n, stride);
 }
 
 __device__ void rows_sum(const RkArgs &A, int64_t base, int64_t r1)

@@ -229,4 +229,196 @@ __device__ __forceinline__ bool controller(StepCtl &c, const double E[4], double
     return done;
 }
 
+__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p)
+{
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ unsigned atom_add_acq_rel_u32(unsigned *p, unsigned x)
+{
+    unsigned old;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(x) : "memory");
+    return old;
+}
+
+__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long k)
+{
+    const unsigned hi = (unsigned)(k >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)k : 0u);
+    return ((unsigned long long)mh << 32) | ml;
+}
+
+// NaN-propagating max of four values that are >= 0 or +NaN over the `parties` CTAs that
+// step one fault (the whole grid in k_rk_step), in one phase.  Every CTA folds its block maximum into a result slot with 64-bit
+// atomicMax on the bit patterns (for such values the unsigned order of the
+// bits is the order of the values, and +NaN lies above +inf, so the fold is
+// nanmax), then arrives on bar with acquire-release semantics; a CTA goes on
+// once bar reaches (attempt + 1) * parties and reads the slot.  Attempts
+// rotate over three slots of four: the CTA that arrives last at attempt a
+// clears slot (a + 2) % 3, which every CTA finished reading before it arrived
+// at a and which no CTA touches before the next barrier.  The last CTA to
+// finish the step clears bar and the slots.  All CTAs return the same four
+// values.  Bounded spin: on timeout ctrl[4] = PQ3D_ERR_TIMEOUT and false is
+// returned.
+template <int NT>
+__device__ __forceinline__ bool fault_max4(double *v, unsigned long long *slots3, unsigned *bar, unsigned parties,
+                                           int attempt, double *ctrl)
+{
+    static_assert(NT == 256, "eight warps: lane 8 q + w reduces maximum q of warp w");
+    __shared__ unsigned long long wred[4][NT / 32];
+    __shared__ double s_res[4];
+    __shared__ int s_ok;
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const unsigned long long m = warp_max_u64((unsigned long long)__double_as_longlong(v[q]));
+        if (lane == 0) wred[q][threadIdx.x >> 5] = m;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        unsigned long long *r = slots3 + 4 * (attempt % 3);
+        unsigned long long m = wred[lane >> 3][lane & 7];
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) {
+            const unsigned long long x = __shfl_xor_sync(0xffffffffu, m, o);
+            m = x > m ? x : m;
+        }
+        if ((lane & 7) == 0) atomicMax(r + (lane >> 3), m);
+        __syncwarp();
+        if (lane == 0) {
+            const unsigned target = (unsigned)(attempt + 1) * parties;
+            int ok = 1;
+            if (atom_add_acq_rel_u32(bar, 1u) + 1u == target) {
+                unsigned long long *z = slots3 + 4 * ((attempt + 2) % 3);
+                for (int e = 0; e < 4; ++e) __stcg(z + e, 0ull);
+            } else {
+                long long it = 0;
+                while (ld_acquire_u32(bar) < target) {
+                    if (++it > (1LL << 24)) {
+                        ctrl[4] = (double)PQ3D_ERR_TIMEOUT;
+                        ok = 0;
+                        break;
+                    }
+                    __nanosleep(32);
+                }
+            }
+            s_ok = ok;
+        }
+        __syncwarp();
+        if (lane < 4) s_res[lane] = __longlong_as_double((long long)__ldcg(r + lane));
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = s_res[q];
+    return s_ok != 0;
+}
+
+// One time step after the load, by each of the fault's CTAs: elements first, first + stride, ...
+// below end per thread, attempts from size c.h until the controller ends the step, state update.
+// F gives what the CTAs of the fault share: ctrl(), hist() and ctrl_host() (may be null), slots3()
+// (3 x 4 error maxima, then 2 slip-rate maxima), bar() and end() (arrivals of the attempts, CTAs
+// done with the step), parties() (CTAs of the fault, all co-resident).  Words zeroed once, cleared
+// by the last CTA.  Functions, and end in the type of the caller: as a struct of pointers formed up
+// front with a 64-bit end, k_rk_step was 0.7 us slower at every size.
+template <int NT, class A_, class F_, class I>
+__device__ __forceinline__ void step_fault(const A_ &A, const F_ &F, StepCtl c, bool forced, int64_t first, I end,
+                                           int64_t stride)
+{
+    double E[4];
+
+    while (true) {
+        double m1 = 0.0, g1 = 0.0, g2 = 0.0, g3 = 0.0;  // max relative errors, NaN-propagating
+        for (int64_t i = first; i < end; i += stride) {
+            double e[4];
+            dp54_element(A, i, c.h, e);
+            m1 = nanmax(m1, e[0]);
+            g1 = nanmax(g1, e[1]);
+            g2 = nanmax(g2, e[2]);
+            g3 = nanmax(g3, e[3]);
+        }
+        // maxima over the fault of (m1, g1, g2, g3); identical in every CTA
+        E[0] = m1; E[1] = g1; E[2] = g2; E[3] = g3;
+        if (!fault_max4<NT>(E, F.slots3(), F.bar(), F.parties(), c.attempt, F.ctrl())) return;
+        if (controller_decide(c, E, A.reltol, forced)) break;
+    }
+    const double h = c.h;
+    // the size after this step: two powers, by a thread of the last warp (idle when R <= 224)
+    // while the others update the state
+    __shared__ double s_next;
+    if (threadIdx.x == NT - 1 && c.accepted) s_next = controller_next(h, E, A.reltol);
+    const bool accepted = c.accepted;
+    const int nrjct = c.nrjct, attempt = c.attempt;
+
+    // accepted step: state update (src/QDsim.py:960-993) and next deficit (:902-903)
+    double mv1 = 0.0, mv2 = 0.0;
+    if (accepted) {
+        for (int64_t i = first; i < end; i += stride) {
+            double v1, v2;
+            accept_element(A, i, h, v1, v2);
+            mv1 = fmax(mv1, fabs(v1));
+            mv2 = fmax(mv2, fabs(v2));
+        }
+    }
+    __shared__ unsigned long long vred[2][NT / 32];
+    {
+        // >= 0 and never NaN: ordered bits
+        const unsigned long long m1 = warp_max_u64((unsigned long long)__double_as_longlong(mv1)),
+                                 m2 = warp_max_u64((unsigned long long)__double_as_longlong(mv2));
+        if ((threadIdx.x & 31) == 0) {
+            vred[0][threadIdx.x >> 5] = m1;
+            vred[1][threadIdx.x >> 5] = m2;
+        }
+    }
+    __syncthreads();
+    // every CTA folds its slip-rate maxima (>= 0, never NaN) into two words; the last one to
+    // finish the step updates ctrl, read ahead of its arrival
+    if (threadIdx.x == 0) {
+        unsigned long long u1 = vred[0][0], u2 = vred[1][0];
+#pragma unroll
+        for (int k = 1; k < NT / 32; ++k) {
+            u1 = vred[0][k] > u1 ? vred[0][k] : u1;
+            u2 = vred[1][k] > u2 ? vred[1][k] : u2;
+        }
+        const double c2 = F.ctrl()[2], c4 = F.ctrl()[4], c8 = F.ctrl()[8], c9 = F.ctrl()[9], c10 = F.ctrl()[10];
+        atomicMax(F.slots3() + 12, u1);
+        atomicMax(F.slots3() + 13, u2);
+        __threadfence();
+        if (atomicAdd(F.end(), 1u) != F.parties() - 1) return;
+        __threadfence();
+        const double w1 = __longlong_as_double((long long)__ldcg(F.slots3() + 12));
+        const double w2 = __longlong_as_double((long long)__ldcg(F.slots3() + 13));
+        *F.end() = 0u;
+        *F.bar() = 0u;
+        for (int q = 0; q < 14; ++q) F.slots3()[q] = 0ull;
+        if (accepted) {
+            const double t = c2 + h, dtnext = s_next;
+            F.ctrl()[2] = t;
+            F.ctrl()[0] = dtnext;   // next dttry
+            F.ctrl()[1] = h;        // accepted step
+            F.ctrl()[3] = nrjct;
+            F.ctrl()[5] = w1;
+            F.ctrl()[6] = w2;
+            F.ctrl()[8] = c8 + 1.0;
+            F.ctrl()[9] = c9 + nrjct;
+            F.ctrl()[10] = c10 + attempt;
+            if (F.hist()) {
+                double *hh = F.hist();
+                hh[0] = h; hh[1] = dtnext; hh[2] = t; hh[3] = w1; hh[4] = w2; hh[5] = nrjct;
+            }
+        } else {
+            F.ctrl()[1] = h;
+            F.ctrl()[3] = nrjct;
+            if (c4 == 0.0) F.ctrl()[4] = (double)PQ3D_ERR_DT;
+        }
+        if (F.ctrl_host()) {
+            // the host's copy, sequence number last (a step that ended early leaves it stale)
+            for (int k = 0; k < 11; ++k) F.ctrl_host()[k] = F.ctrl()[k];
+            __threadfence_system();
+            F.ctrl_host()[15] = (double)A.step_index + 1.0;
+        }
+    }
+}
+
 }  // namespace pq3d_rk

@@ -151,8 +151,9 @@ class Ensemble:
                        vplc=lambda s: s.slipvC, cr0=lambda s: np.cos(s.rake0), sr0=lambda s: np.sin(s.rake0))
         self.t = {k: torch.tensor(np.ascontiguousarray(cat(g)), **f64) for k, g in getters.items()}
         # tasks as short as gives half the co-resident grid a task (in 16s), so that a small
-        # ensemble's row sums and element work spread over all SMs (12.6k elements: 28 us per
-        # step kernel with 96 rows, 33 with 256)
+        # ensemble's row sums and element work spread over all SMs, and all tasks get a CTA of
+        # their own (12.6k elements: 19.0 us per step kernel with 96 rows, 22.2 with 256; 44 in
+        # lock step with 32, more tasks than CTAs)
         cap = max(1, self.L.pq3d_ens_grid(1 << 30) // 2)
         rows = min(self.L.pq3d_ens_task_rows(), 16 * -(-n // (16 * cap)))
         task_row, task_fault, fault_task = ensemble_tasks(self.struct.row0, rows)
@@ -167,7 +168,7 @@ class Ensemble:
         self.cand = torch.zeros(4 * n, **f64)
         self.tmax = torch.zeros(4 * T, **f64)
         self.ctrl = torch.zeros((M, 16), **f64)
-        self.fstate = torch.zeros((M, 8), **f64)
+        self.fstate = torch.zeros((M, 24), **f64)
         self.bar = torch.zeros(4, dtype=torch.int32, device=dev)
         self.hist = None
         self.hist_cap = 0
