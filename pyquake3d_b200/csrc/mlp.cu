@@ -11,9 +11,9 @@
 //                 the Adam update
 // Bound: 24.6 kFLOP a sample in FP32 (100 MFLOP = 1.4 us for 4,096 samples); the batch has
 // to be spread over the SMs, since each layer is a chain of 64 dependent FMAs.  B = 4,096 on
-// B200: 11.4 + 3.4 us, against 110 + 55 + 14 + 2 us for separate forward, backward, weight
+// B200: 8.4 + 3.4 us, against 110 + 55 + 14 + 2 us for separate forward, backward, weight
 // gradient and Adam kernels with one thread a sample (32 CTAs, the hidden vector in local
-// memory, activations through HBM); an epoch of 65,536 samples 3.42 -> 0.45 ms.
+// memory, activations through HBM); an epoch of 65,536 samples 3.42 -> 0.42 ms.
 #include "pq3d_common.cuh"
 #include <math.h>
 
@@ -35,16 +35,29 @@ struct Weights {
 // Thread roles.  Layer 1: sample = lane, units 8 * warp + 0..7.  Layers 2 and 3 and the
 // backward product: units u0 = 8 * warp + 4 * (lane / 16) + 0..3, samples 2 * (lane % 16) + 0..1
 // (per column of W2: one broadcast 16-byte and one 8-byte shared load for eight FMAs).
+// All loads of a thread in flight at once, then the stores: in loops they were eight round trips
+// to L2, 8,800 of the gradient kernel's 20,000 cycles (11.4 -> 8.4 us).  Scalar, since P has any
+// alignment.
 __device__ __forceinline__ void load_weights(Weights &w, const float *__restrict__ P)
 {
-    for (int e = threadIdx.x; e < H * H; e += MT) w.W2[(e >> 6) * WST + (e & 63)] = P[OFF_W2 + e];
-    for (int e = threadIdx.x; e < H * NIN; e += MT) w.W1[e] = P[OFF_W1 + e];
-    if (threadIdx.x < H) {
-        w.b1[threadIdx.x] = P[OFF_B1 + threadIdx.x];
-        w.b2[threadIdx.x] = P[OFF_B2 + threadIdx.x];
-        w.W3[threadIdx.x] = P[OFF_W3 + threadIdx.x];
+    static_assert(OFF_B1 + H <= 2 * MT && NP - OFF_B2 <= MT, "W1, b1 in two loads; b2, W3, b3 in one");
+    const int t = threadIdx.x;
+    float q[H * H / MT];
+#pragma unroll
+    for (int k = 0; k < H * H / MT; ++k) q[k] = P[OFF_W2 + k * MT + t];
+    const float head0 = P[OFF_W1 + t], head1 = MT + t < OFF_W2 ? P[OFF_W1 + MT + t] : 0.0f;
+    const float tail = OFF_B2 + t < NP ? P[OFF_B2 + t] : 0.0f;
+#pragma unroll
+    for (int k = 0; k < H * H / MT; ++k) {
+        const int e = k * MT + t;
+        w.W2[(e >> 6) * WST + (e & 63)] = q[k];
     }
-    if (threadIdx.x == 0) w.b3 = P[OFF_B3];
+    w.W1[t] = head0;
+    if (MT + t < OFF_B1) w.W1[MT + t] = head1;
+    else if (MT + t < OFF_W2) w.b1[MT + t - OFF_B1] = head1;
+    if (t < H) w.b2[t] = tail;
+    else if (t < 2 * H) w.W3[t - H] = tail;
+    else if (t == 2 * H) w.b3 = tail;
 }
 
 // Samples b0.. of X (0 beyond B) into xs[sample][NIN].
@@ -170,6 +183,8 @@ __global__ void __launch_bounds__(MT, 2) k_mlp_grad(const float *__restrict__ P,
     load_weights(w, P);
     for (int64_t b0 = (int64_t)blockIdx.x * TS; b0 < B; b0 += (int64_t)gridDim.x * TS) {
         load_tile(xs, X, xstride, (int)b0, B);
+        const bool mine = threadIdx.x < TS && b0 + threadIdx.x < B;
+        const float target = mine ? T[(b0 + threadIdx.x) * tstride] : 0.0f;   // ahead of its use
         __syncthreads();
         layer1(w, xs, h1);
         __syncthreads();
@@ -179,8 +194,8 @@ __global__ void __launch_bounds__(MT, 2) k_mlp_grad(const float *__restrict__ P,
         __syncthreads();
         if (threadIdx.x < TS) {
             float d3 = 0.0f;
-            if (b0 + threadIdx.x < B) {
-                const float r = output_sum(w, yp, threadIdx.x) - T[(b0 + threadIdx.x) * tstride];
+            if (mine) {
+                const float r = output_sum(w, yp, threadIdx.x) - target;
                 d3 = r / (float)B;
                 gl += 0.5f * r * r / (float)B;
             }
