@@ -30,6 +30,7 @@ import struct as _struct
 import numpy as np
 
 from . import _lib
+from .hmatrix import workspace_table
 
 MAGIC = b"PQ3DOP\x00\x01"
 VERSION = 1
@@ -150,7 +151,7 @@ def load_operator(op, path, xg, ev):
     op.dense64 = torch.from_numpy(d64).to(op.dev) if d64 is not None else None
     op.dense32 = torch.from_numpy(d32).to(op.dev) if d32 is not None else None
     op.aca_ws = []
-    op.task_ws = {}
+    op.task_ws = workspace_table(0)
     for d in header["precisions"]:
         U, V = _read(path, header, "U_" + d), _read(path, header, "V_" + d)
         if d == "mixed":

@@ -245,6 +245,12 @@ def _fields(dtype, n, **cols):
     return rec
 
 
+def workspace_table(ntasks):
+    """Where every ACA task's factors are: workspace, offset in it and room for terms (none:
+    ntasks 0, as an operator read from a checkpoint has it)."""
+    return {k: np.zeros(ntasks, np.int64) for k in ("ws", "off", "kmax")}
+
+
 def _block_geometry(blocks):
     """(m, n, first row, first column, lo, hi) of blocks in tree order; [lo, hi) are the
     block-local rows the plan computes (all, unless a row partition clipped them)."""
@@ -867,7 +873,7 @@ class DeviceHMatrix:
         self.aca_ranks = np.zeros(nt, dtype=np.int32)
         self.aca_flags = np.zeros(nt, dtype=np.int32)
         self.aca_ws = []                         # workspaces; a task's is task_ws["ws"][task]
-        self.task_ws = {k: np.zeros(nt, np.int64) for k in ("ws", "off", "kmax")}
+        self.task_ws = workspace_table(nt)
         kcap = np.minimum(np.minimum(m, n), self.kcap)
         pending = np.arange(nt)
         while len(pending):
