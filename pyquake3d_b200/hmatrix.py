@@ -245,6 +245,14 @@ def _fields(dtype, n, **cols):
     return rec
 
 
+def _check32(**sizes):
+    """The records hold these in 32 bits, and an assignment to a column wraps silently: refuse a
+    plan beyond that before its items are made."""
+    for k, v in sizes.items():
+        if v > 0x7fffffff:
+            raise OverflowError("%s of the plan: %d does not fit the work items' 32 bits" % (k, v))
+
+
 def workspace_table(ntasks):
     """Where every ACA task's factors are: workspace, offset in it and room for terms (none:
     ntasks 0, as an operator read from a checkpoint has it)."""
@@ -301,6 +309,7 @@ def build_plan_arrays(struct, dense_recs, kS, kD, code, dense_chunk=64, v_chunk=
     tp, n_tpart = _offsets(nch * Q)
     slot, n_slots = _offsets(hi - lo)
     slot, n_slots = slot + slot0, n_slots + slot0
+    _check32(slots=n_slots, t_positions=n_tpart)
     # V items: per column chunk, the strike rows then the dip rows, 32 to an item
     nS, nD = _cdiv(3 * ks, 32), _cdiv(3 * kd, 32)
     b, i = _expand(nch * (nS + nD))
@@ -343,6 +352,7 @@ def _dense_items(dense_recs, cwd, dense_off, dense_chunk):
     nch, nr = _cdiv(ng, dense_chunk), _cdiv(m, 32)
     ob, ch = _expand(nch)                              # slot owners: (block, column chunk)
     slot, n_slots = _offsets(m[ob])
+    _check32(slots=n_slots)
     o, i = _expand(nr[ob])
     b = ob[o]
     ditems = np.zeros(len(o), dtype=_lib.DENSE_ITEM)
@@ -493,6 +503,7 @@ def build_plan_arrays_mixed(struct, dense_recs, cls_lists, dense_chunk=16, v_chu
     tp, sb = np.where(K > 0, tp.reshape(-1, 3), 0), np.where((K > 0) & (np.arange(3) > 0), sb.reshape(-1, 3), 0)
     slot, n_slots = _offsets(hi - lo)
     slot, n_slots = slot + slot0, n_slots + slot0
+    _check32(slots=n_slots, t_positions=n_tpart, scales=n_scales, row_stride=int((Q * CW).max(initial=0)))
     # one entry per (block, class) with rows, for the merged V items
     b, c = np.nonzero(K > 0)
     vitems, vwarp, vrows = _merged_v_items(c0[b], nn[b], c, v_off[b, c], Q[b, c], 3 * ks[b, c], tp[b, c], v_chunk,

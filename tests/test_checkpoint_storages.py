@@ -1,6 +1,6 @@
 """An operator without low-rank blocks read back from a checkpoint takes further storages:
-its FP32 near field serves the FP32, BF16 and FP32-dense mixed plans, with no factors to
-pack.  CPU: the operator object holds host tensors and launches nothing on this path."""
+its FP32 near field serves the FP32 and BF16 plans, with no factors to pack.  CPU: the
+operator object holds host tensors and launches nothing on this path."""
 import numpy as np
 import pytest
 
