@@ -48,8 +48,9 @@ def test_t_positions(code):
 
 
 def test_t_positions_mixed():
+    # a V class array has four or more entries per t position: its own limit comes first
     s = _struct(8, 2 ** 16, 4)
-    with pytest.raises(OverflowError):
+    with pytest.raises(_lib.Pq3dError):
         build_plan_arrays_mixed(s, _no_dense(), None, v_chunk=1, counts=np.full((4, 2, 3), 2 ** 14))
 
 
