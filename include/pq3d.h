@@ -233,13 +233,17 @@ int pq3d_rk_rows_finish(double *d_pc, const double *d_V8, cudaStream_t stream);
  * controller.  Rows of a fault are a contiguous tree-order range; CTA tasks of
  * at most pq3d_ens_task_rows() rows never span two faults.  ctrl holds 16
  * doubles per fault (layout of the pq3d_rk_step control block), hist 6 doubles
- * per (step, fault), fstate 24 doubles per fault, zeroed once.  With as many
- * CTAs as tasks each fault steps on its own; with fewer the faults advance in
- * lock-step attempts. */
+ * per (step, fault), fstate 8 doubles per fault.
+ * pq3d_ens_step: the faults advance in lock-step attempts, with any co-resident
+ * grid.  pq3d_ens_step_faults: a CTA per task (pq3d_ens_grid(n_tasks) ==
+ * n_tasks), each fault on its own; d_meet pq3d_ens_meet_bytes(n_faults) bytes,
+ * zeroed once (every step leaves them cleared). */
 size_t pq3d_ens_args_bytes(void);
 int pq3d_ens_task_rows(void);
 int pq3d_ens_grid(int n_tasks);
 int pq3d_ens_step(const void *args, int grid, cudaStream_t stream);
+size_t pq3d_ens_meet_bytes(int n_faults);
+int pq3d_ens_step_faults(const void *args, void *d_meet, cudaStream_t stream);
 
 /* ---------------------------------------------------------------- V-mode and MLP
  * No counterpart in the reference: slip and state integrated with DP5(4), one

@@ -147,10 +147,13 @@ def load():
     L.pq3d_ens_args_bytes.restype = ctypes.c_size_t
     L.pq3d_ens_grid.argtypes = [i32]
     L.pq3d_ens_step.argtypes = [vp, i32, vp]
+    L.pq3d_ens_step_faults.argtypes = [vp, vp, vp]
+    L.pq3d_ens_meet_bytes.argtypes = [i32]
+    L.pq3d_ens_meet_bytes.restype = ctypes.c_size_t
     for f in ("pq3d_src_records", "pq3d_hs_records", "pq3d_traction_pairs", "pq3d_stress_points", "pq3d_dense_assemble",
               "pq3d_aca_batched", "pq3d_aca_pack", "pq3d_hmatvec", "pq3d_nearfield_rowabs", "pq3d_aca_term_weights",
               "pq3d_aca_pack_mixed", "pq3d_rk_grid", "pq3d_rk_step", "pq3d_ens_grid",
-              "pq3d_ens_step", "pq3d_ens_task_rows", "pq3d_rk_rows_attempt", "pq3d_rk_rows_accept",
+              "pq3d_ens_step", "pq3d_ens_step_faults", "pq3d_ens_task_rows", "pq3d_rk_rows_attempt", "pq3d_rk_rows_accept",
               "pq3d_rk_rows_attempt_dev", "pq3d_rk_rows_control", "pq3d_rk_rows_accept_dev", "pq3d_rk_rows_finish",
               "pq3d_host_map_alloc", "pq3d_host_map_free", "pq3d_event_create", "pq3d_event_destroy",
               "pq3d_event_record", "pq3d_event_sync", "pq3d_event_query", "pq3d_snapshot", "pq3d_stream_wait_event"):

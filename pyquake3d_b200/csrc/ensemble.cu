@@ -7,7 +7,7 @@
 // (the reference's simu_forward after the load, src/QDsim.py:892-996): DP5(4)
 // attempts with the frozen load, NaN-propagating error maxima over the fault's
 // elements, the reference controller, and the accepted-step update.  With a CTA per task
-// (k_rk_faults) each fault runs on its own; with several tasks per CTA (k_rk_ensemble) faults
+// (k_rk_faults) each fault runs on its own; with any number of CTAs (k_rk_ensemble) faults
 // advance in lock-step attempts, and one whose step is accepted (or given up) is skipped by
 // the later attempts of the others.
 //
@@ -25,8 +25,8 @@ using namespace pq3d_rk;
 
 constexpr int ENS_THREADS = 256;
 constexpr int ENS_CTRL = 16;    // doubles of per-fault control (layout of the single-fault ctrl)
-constexpr int ENS_FSTATE = 24;  // doubles of per-fault scratch: attempt state of the lock-step kernel, and
-constexpr int ENS_WORDS = 8;    // from here on the 14 + 1 words a fault's CTAs meet at
+constexpr int ENS_FSTATE = 8;   // doubles of per-fault attempt state (lock step)
+constexpr int ENS_MEET = 16;    // 8-byte words at which the CTAs of a fault on its own meet: 14 + 1 used
 constexpr int ENS_MAX_ATTEMPTS = 64;
 
 struct EnsArgs {
@@ -43,8 +43,7 @@ struct EnsArgs {
     const int32_t *fault_task; // tasks of fault s: [fault_task[s], fault_task[s+1])
     double *tmax;              // 4 doubles per task
     double *ctrl;              // ENS_CTRL doubles per fault
-    double *fstate;            // ENS_FSTATE doubles per fault: h, dtnext, nrjct, attempt, phase; meeting
-                               // words at ENS_WORDS (zeroed once)
+    double *fstate;            // ENS_FSTATE doubles per fault: h, dtnext, nrjct, attempt, phase
     double *hist;              // 6 doubles per (step, fault), may be null
     const double *hforce;      // dt replay: step s of fault f takes hforce[s * n_faults + f]
     unsigned *bar;             // [0] arrivals, [1] generation, [2] end-of-step count, [3] all-done flag
@@ -281,14 +280,12 @@ __global__ void __launch_bounds__(ENS_THREADS) k_rk_ensemble(EnsArgs A)
 
 struct OneFault {
     const EnsArgs &A;
+    unsigned long long *meet;   // the fault's words
     int s;
     __device__ double *ctrl() const { return A.ctrl + (int64_t)ENS_CTRL * s; }
     __device__ double *hist() const { return A.hist ? A.hist + 6 * ((int64_t)A.step_index * A.n_faults + s) : nullptr; }
     __device__ double *ctrl_host() const { return nullptr; }
-    __device__ unsigned long long *slots3() const
-    {
-        return (unsigned long long *)(A.fstate + (int64_t)ENS_FSTATE * s + ENS_WORDS);
-    }
+    __device__ unsigned long long *slots3() const { return meet; }
     __device__ unsigned *bar() const { return (unsigned *)(slots3() + 14); }
     __device__ unsigned *end() const { return bar() + 1; }
     __device__ unsigned parties() const { return (unsigned)(A.fault_task[s + 1] - A.fault_task[s]); }
@@ -298,7 +295,7 @@ struct OneFault {
 // another's attempts, the maxima are folded in one phase and the next size is computed beside the
 // state update.  B200, six faults, 12.6k elements: 18.9 us a launch, 28.1 in lock step.
 template <typename TA>
-__global__ void __launch_bounds__(ENS_THREADS, 2) k_rk_faults(EnsArgs A)
+__global__ void __launch_bounds__(ENS_THREADS, 2) k_rk_faults(EnsArgs A, unsigned long long *meet)
 {
     const int t = blockIdx.x, s = A.task_fault[t];
     const int64_t r0 = A.task_row[t], r1 = A.task_row[t + 1];
@@ -306,7 +303,7 @@ __global__ void __launch_bounds__(ENS_THREADS, 2) k_rk_faults(EnsArgs A)
     const bool forced = A.hforce != nullptr;
     const double h = forced ? A.hforce[(int64_t)A.step_index * A.n_faults + s] : A.ctrl[(int64_t)ENS_CTRL * s];
     const StepCtl c{h, 0.0, 0, 0, false};
-    step_fault<ENS_THREADS>(A, OneFault{A, s}, c, forced, r0 + threadIdx.x, r1, ENS_THREADS);
+    step_fault<ENS_THREADS>(A, OneFault{A, meet + (int64_t)ENS_MEET * s, s}, c, forced, r0 + threadIdx.x, r1, ENS_THREADS);
 }
 
 }  // namespace
@@ -334,15 +331,24 @@ PQ3D_EXPORT int pq3d_ens_grid(int n_tasks)
 // Rows per ensemble task (tasks never span two faults).
 PQ3D_EXPORT int pq3d_ens_task_rows(void) { return ENS_THREADS; }
 
-// One time step of every fault of the ensemble (cooperative launch).
-PQ3D_EXPORT int pq3d_ens_step(const void *args, int grid, cudaStream_t stream)
+// Bytes of the words at which the CTAs of faults on their own meet.
+PQ3D_EXPORT size_t pq3d_ens_meet_bytes(int n_faults)
 {
-    if (!args || grid <= 0) return PQ3D_ERR_ARG;
-    EnsArgs A = *(const EnsArgs *)args;
+    return n_faults > 0 ? (size_t)n_faults * ENS_MEET * sizeof(unsigned long long) : 0;
+}
+
+static int ens_check(const EnsArgs &A)
+{
     if (A.n <= 0 || A.n_faults <= 0 || A.n_tasks <= 0 || !A.task_row || !A.task_fault || !A.fault_task ||
         !A.tmax || !A.ctrl || !A.fstate || !A.bar || !A.y || !A.cand || !A.x)
         return PQ3D_ERR_ARG;
     if (A.fuse_rowsum && (!A.slots || !A.leaf_of_row || !A.leaf_ptr || !A.leaf_off)) return PQ3D_ERR_ARG;
+    return PQ3D_OK;
+}
+
+template <class K, class... P>
+static int ens_launch(K kernel, int grid, cudaStream_t stream, const P &...params)
+{
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(ENS_THREADS);
@@ -352,11 +358,28 @@ PQ3D_EXPORT int pq3d_ens_step(const void *args, int grid, cudaStream_t stream)
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    // a CTA per task needs every task co-resident; above that (75k rows at 256 a task, or more
-    // faults than CTAs) the CTAs take several tasks each, in lock step
-    if (grid == A.n_tasks)
-        PQ3D_CHECK(cudaLaunchKernelEx(&cfg, A.slots_fp32 ? k_rk_faults<float> : k_rk_faults<double>, A));
-    else
-        PQ3D_CHECK(cudaLaunchKernelEx(&cfg, A.slots_fp32 ? k_rk_ensemble<float> : k_rk_ensemble<double>, A));
+    PQ3D_CHECK(cudaLaunchKernelEx(&cfg, kernel, params...));
     return PQ3D_OK;
+}
+
+// One time step of every fault of the ensemble (cooperative launches): in lock step, with any
+// grid; or each fault on its own, with a CTA per task (all co-resident).  Two entries, since the
+// second needs the meeting words, which a caller of the first has not got.
+PQ3D_EXPORT int pq3d_ens_step(const void *args, int grid, cudaStream_t stream)
+{
+    if (!args || grid <= 0) return PQ3D_ERR_ARG;
+    const EnsArgs A = *(const EnsArgs *)args;
+    const int rc = ens_check(A);
+    if (rc != PQ3D_OK) return rc;
+    return ens_launch(A.slots_fp32 ? k_rk_ensemble<float> : k_rk_ensemble<double>, grid, stream, A);
+}
+
+PQ3D_EXPORT int pq3d_ens_step_faults(const void *args, void *d_meet, cudaStream_t stream)
+{
+    if (!args || !d_meet) return PQ3D_ERR_ARG;
+    const EnsArgs A = *(const EnsArgs *)args;
+    const int rc = ens_check(A);
+    if (rc != PQ3D_OK) return rc;
+    return ens_launch(A.slots_fp32 ? k_rk_faults<float> : k_rk_faults<double>, A.n_tasks, stream, A,
+                      (unsigned long long *)d_meet);
 }

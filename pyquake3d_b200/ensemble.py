@@ -168,7 +168,8 @@ class Ensemble:
         self.cand = torch.zeros(4 * n, **f64)
         self.tmax = torch.zeros(4 * T, **f64)
         self.ctrl = torch.zeros((M, 16), **f64)
-        self.fstate = torch.zeros((M, 24), **f64)
+        self.fstate = torch.zeros((M, 8), **f64)
+        self.meet = torch.zeros(self.L.pq3d_ens_meet_bytes(M) // 8, dtype=torch.int64, device=dev)
         self.bar = torch.zeros(4, dtype=torch.int32, device=dev)
         self.hist = None
         self.hist_cap = 0
@@ -206,7 +207,11 @@ class Ensemble:
         if self.hforce is not None and step_index >= self.hforce_cap:
             raise _lib.Pq3dError("dt replay shorter than the run")
         self.args["hforce"] = self.hforce.data_ptr() if self.hforce is not None else 0
-        check(self.L.pq3d_ens_step(self.args.ctypes.data, self.grid, _lib.stream_ptr(stream)), "pq3d_ens_step")
+        st = _lib.stream_ptr(stream)
+        if self.grid == self.n_tasks:       # a CTA per task: each fault on its own, else in lock step
+            check(self.L.pq3d_ens_step_faults(self.args.ctypes.data, ptr(self.meet), st), "pq3d_ens_step_faults")
+        else:
+            check(self.L.pq3d_ens_step(self.args.ctypes.data, self.grid, st), "pq3d_ens_step")
 
     def set_history(self, nsteps):
         self.hist = self.torch.zeros((max(nsteps, 1), self.M, 6), dtype=self.torch.float64, device=self.op.dev)
