@@ -59,9 +59,9 @@ __device__ __forceinline__ void rowsum_rows(const TA *__restrict__ slots, const 
         k = leaf_ptr[l] + g;
         k1 = leaf_ptr[l + 1];
     }
-    // leaves are numbered in row order: the CTA's lists are one range of leaf_off
+    // with leaves numbered in row order the CTA's lists are one range of leaf_off
     const int kb = leaf_ptr[leaf_of_row[base]], ke = leaf_ptr[leaf_of_row[base + rows - 1] + 1];
-    const bool staged = ke - kb <= RS_STAGE;
+    const bool staged = (unsigned)(ke - kb) <= (unsigned)RS_STAGE;      // ke < kb: another numbering
     __syncthreads();             // s_off and s_part of the CTA's previous rows are no longer read
     if (staged)
         for (int e = kb + (int)threadIdx.x; e < ke; e += NT) s_off[e - kb] = __ldg(leaf_off + e);
@@ -103,7 +103,8 @@ __device__ __forceinline__ void rowsum_rows(const TA *__restrict__ slots, const 
             k = kn;
         }
     };
-    if (staged) sum([&](int e) { return s_off[e - kb]; });
+    // a list outside the range, which another numbering of the leaves has, is read in place
+    if (staged && k >= kb && k1 <= ke) sum([&](int e) { return s_off[e - kb]; });
     else sum([&](int e) { return __ldg(leaf_off + e); });
     if (G == 1) {
         if (g == 0 && r < rows) emit(r, a);      // threads R.. NT have no row (R = 208: 48 of them)
