@@ -120,9 +120,12 @@ __device__ void cta_max4(double *v, double *out)
     __syncthreads();
 }
 
-// TA: type of the matvec's slots.
+// TA: type of the matvec's slots.  The last CTA's walk over the faults, some 3 us for every eight,
+// is most of it.  Straight-line stages and whole CTAs on a task's rows: 320 faults of 56 rows
+// 169 us a step, 800 of 20 373 (180 and 400 with the step kernel's rolled stages, short groups and
+// one thread counting the faults that go on).
 template <typename TA>
-__global__ void __launch_bounds__(ENS_THREADS) k_rk_ensemble(EnsArgs A)
+__global__ void __launch_bounds__(ENS_THREADS, 2) k_rk_ensemble(EnsArgs A)
 {
     __shared__ unsigned s_gen;
     __shared__ int s_last;
@@ -143,12 +146,12 @@ __global__ void __launch_bounds__(ENS_THREADS) k_rk_ensemble(EnsArgs A)
             // the H-matvec's row sums of the task's rows (one task is at most ENS_THREADS rows)
             if (k == 0 && A.fuse_rowsum) {
                 const int r0 = A.task_row[t], r1 = A.task_row[t + 1];
-                rowsum_cta<ENS_THREADS, TA>(A, r0, r1, (r1 - r0 + 15) & ~15);
+                rowsum_cta<ENS_THREADS, TA>(A, r0, r1, ENS_THREADS);
             }
             double e4[4] = {0.0, 0.0, 0.0, 0.0};
             for (int64_t i = A.task_row[t] + threadIdx.x; i < A.task_row[t + 1]; i += ENS_THREADS) {
                 double e[4];
-                dp54_element(A, i, h, e);
+                dp54_element<true>(A, i, h, e);
 #pragma unroll
                 for (int q = 0; q < 4; ++q) e4[q] = nanmax(e4[q], e[q]);
             }
@@ -159,6 +162,7 @@ __global__ void __launch_bounds__(ENS_THREADS) k_rk_ensemble(EnsArgs A)
         // last CTA: per-fault maxima and controller
         if (arrive(A.bar, &s_gen, &s_last)) {
             const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+            int open = 0;                       // a fault of this warp goes on
             for (int s = warp; s < M; s += ENS_THREADS / 32) {
                 double *fs = A.fstate + (int64_t)ENS_FSTATE * s;
                 StepCtl c;
@@ -184,6 +188,7 @@ __global__ void __launch_bounds__(ENS_THREADS) k_rk_ensemble(EnsArgs A)
 #pragma unroll
                     for (int o = 16; o > 0; o >>= 1) E[q] = nanmax(E[q], __shfl_xor_sync(0xffffffffu, E[q], o));
                 const bool done = controller(c, E, A.reltol, forced);
+                open |= !done;
                 if (lane == 0) {
                     fs[0] = c.h;
                     fs[1] = c.dtnext;
@@ -192,13 +197,8 @@ __global__ void __launch_bounds__(ENS_THREADS) k_rk_ensemble(EnsArgs A)
                     fs[4] = done ? (c.accepted ? 1.0 : 2.0) : 0.0;
                 }
             }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                __threadfence();
-                unsigned running = 0;
-                for (int s = 0; s < M; ++s) running += A.fstate[(int64_t)ENS_FSTATE * s + 4] == 0.0;
-                A.bar[3] = running == 0 ? 1u : 0u;
-            }
+            open = __syncthreads_or(open);
+            if (threadIdx.x == 0) A.bar[3] = open ? 0u : 1u;
             release(A.bar);
         } else if (!wait_release(A, s_gen)) {
             return;
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(ENS_THREADS) k_rk_ensemble(EnsArgs A)
         if (acc) {
             for (int64_t i = A.task_row[t] + threadIdx.x; i < A.task_row[t + 1]; i += ENS_THREADS) {
                 double v1, v2;
-                accept_element(A, i, h, v1, v2);
+                accept_element<true>(A, i, h, v1, v2);
                 v4[0] = fmax(v4[0], fabs(v1));
                 v4[1] = fmax(v4[1], fabs(v2));
             }

@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(RK_THREADS) k_rk_rows_attempt(RkArgs A, int r0
             rows_sum(A, base, r1);
     for (int64_t i = r0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < r1; i += stride) {
         double e[4];
-        dp54_element(A, i, h, e);
+        dp54_element<true>(A, i, h, e);
 #pragma unroll
         for (int q = 0; q < 4; ++q) e4[q] = nanmax(e4[q], e[q]);
     }
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(RK_THREADS) k_rk_rows_accept(RkArgs A, int r0,
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = r0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < r1; i += stride) {
         double v1, v2;
-        accept_element(A, i, h, v1, v2);
+        accept_element<true>(A, i, h, v1, v2);
         v4[0] = fmax(v4[0], fabs(v1));
         v4[1] = fmax(v4[1], fabs(v2));
     }
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(RK_THREADS) k_rk_rows_attempt_dev(RkArgs A, in
             rows_sum(A, base, r1);
     for (int64_t i = r0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < r1; i += stride) {
         double e[4];
-        dp54_element(A, i, h, e);
+        dp54_element<true>(A, i, h, e);
 #pragma unroll
         for (int q = 0; q < 4; ++q) e4[q] = nanmax(e4[q], e[q]);
     }
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(RK_THREADS) k_rk_rows_accept_dev(RkArgs A, int
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = r0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < r1; i += stride) {
         double v1, v2;
-        accept_element(A, i, h, v1, v2);
+        accept_element<true>(A, i, h, v1, v2);
         v4[0] = fmax(v4[0], fabs(v1));
         v4[1] = fmax(v4[1], fabs(v2));
     }

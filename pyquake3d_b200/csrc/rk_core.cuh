@@ -81,7 +81,9 @@ __device__ __forceinline__ void rowsum_cta(const A &S, int64_t base, int64_t end
 // src/QDsim.py:1001-1134) with the frozen load y[i] and start-of-step slip rate:
 // the 5th-order candidate goes to cand (Tno, Tt1o, Tt2o, psi planes of n), the
 // relative error terms |dpsi/psi8|, |dTt1/Tt1_8|, |dTt2/Tt2_8|, |dTno/Tno8| to err.
-template <class A>
+// FLAT: straight-line stages.  The step kernels, short CTAs that meet at every attempt, take the
+// rolled form; the row-range and lock-step kernels lose by it (see below).  Same bits.
+template <bool FLAT = false, class A>
 __device__ __forceinline__ void dp54_element(const A &S, int64_t i, double h, double err[4])
 {
     const int64_t n = S.n;
@@ -91,22 +93,24 @@ __device__ __forceinline__ void dp54_element(const A &S, int64_t i, double h, do
     const double L1 = S.y[3 * i], L2 = S.y[3 * i + 1];
     const double dsg = S.fix_tn ? S.normal_loading[i] : S.y[3 * i + 2] + S.normal_loading[i];
     const double y0[4] = {S.Tno[i], S.Tt1o[i], S.Tt2o[i], S.psi[i]};
-    // The stages are one rolled loop with the derivatives in local memory (L1).  Unrolled they
-    // made k_rk_step 124 KB of code (57 KB now) that ran once per attempt, with spills.
+    // Rolled, the stages are one loop with the derivatives in local memory (L1).  Unrolled they made
+    // k_rk_step 124 KB of code (57 KB rolled) that ran once per attempt, with spills.  An attempt of
+    // the row-range kernel, rolled and unrolled, us: 15.2 and 13.2 at 784 rows, 19.1 and 17.1 at 5,120,
+    // 43.8 and 41.3 at 60k.
     double k[7][4], y[4] = {y0[0], y0[1], y0[2], y0[3]};
     auto combine = [&](int s, double *o) {
         double acc[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 1
-        for (int j = 0; j < (s < 7 ? s : 7); ++j) {
+#pragma unroll (FLAT ? 7 : 1)
+        for (int j = 0; j < (FLAT ? 7 : s < 7 ? s : 7); ++j) {
             const double w = kDp[s][j];
-            if (w == 0.0) continue;
+            if (FLAT ? j >= s || (j == 1 && s >= 6) : w == 0.0) continue;      // the tableau's zeros
 #pragma unroll
             for (int q = 0; q < 4; ++q) acc[q] += w * k[j][q];
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) o[q] = y0[q] + h * acc[q];
     };
-#pragma unroll 1
+#pragma unroll (FLAT ? 7 : 1)
     for (int s = 0; s < 7; ++s) {
         if (s > 0) combine(s, y);
         const Deriv d = derivative(y[0], y[1], y[2], y[3], ia, ib, bdc, f0, S.V0, sv, L1, L2, dsg, sh, S.eta);
@@ -129,8 +133,8 @@ __device__ __forceinline__ void dp54_element(const A &S, int64_t i, double h, do
 
 // Accepted step for element i (src/QDsim.py:960-993): state from cand, slip
 // rates, rake, slip, friction, and the next slip-rate deficit in both x layouts
-// (:902-903).  Returns the new slip rates (v1o, v2o).
-template <class A>
+// (:902-903).  Returns the new slip rates (v1o, v2o).  FLAT as above.
+template <bool FLAT = false, class A>
 __device__ __forceinline__ void accept_element(const A &S, int64_t i, double h, double &v1o, double &v2o)
 {
     const int64_t n = S.n;
@@ -141,7 +145,7 @@ __device__ __forceinline__ void accept_element(const A &S, int64_t i, double h, 
     S.Tt[i] = sqrt(T1 * T1 + T2 * T2);
     const double ex = exp(-ps / a);
     double v1 = 0.0, v2 = 0.0;
-#pragma unroll 1
+#pragma unroll (FLAT ? 2 : 1)
     for (int c = 0; c < 2; ++c) {
         const double v = (2.0 * S.V0) * ex * sinh((c ? T2 : T1) / Tn / a);
         (c ? v2 : v1) = v;
@@ -186,11 +190,14 @@ struct StepCtl {
     bool accepted;
 };
 
-// The controller's sizes for error maxima E: the smaller of the two estimates.
+// The controller's sizes for error maxima E: the smaller of the two estimates.  The two powers
+// one after the other (PAIR false: half the code, for the step kernels, where they run beside the
+// state update) or overlapping.
+template <bool PAIR>
 __device__ __forceinline__ double controller_size(double h, const double E[4], double reltol)
 {
     double hnew[2];
-#pragma unroll 1
+#pragma unroll (PAIR ? 2 : 1)
     for (int k = 0; k < 2; ++k) {
         const double R = (k ? py_max(py_max(E[1], E[2]), E[3]) : E[0]) + 1e-10;
         hnew[k] = h * 0.9 * pow(reltol / R, 0.2);
@@ -199,13 +206,15 @@ __device__ __forceinline__ double controller_size(double h, const double E[4], d
 }
 
 // The size after an accepted attempt of size h.
+template <bool PAIR = false>
 __device__ __forceinline__ double controller_next(double h, const double E[4], double reltol)
 {
-    return py_min(controller_size(h, E, reltol), 1.5 * h);
+    return py_min(controller_size<PAIR>(h, E, reltol), 1.5 * h);
 }
 
 // As controller(), but leaves dtnext of an accepted attempt to controller_next (two powers
 // that only the thread that stores it needs).
+template <bool PAIR = false>
 __device__ __forceinline__ bool controller_decide(StepCtl &c, const double E[4], double reltol, bool forced)
 {
     const double R1 = E[0] + 1e-10;
@@ -217,15 +226,15 @@ __device__ __forceinline__ bool controller_decide(StepCtl &c, const double E[4],
         return true;
     }
     c.nrjct++;
-    c.dtnext = controller_size(c.h, E, reltol);
+    c.dtnext = controller_size<PAIR>(c.h, E, reltol);
     c.h = py_max(0.5 * c.h, c.dtnext);
     return c.h < 1.e-15 || c.nrjct > 20;
 }
 
 __device__ __forceinline__ bool controller(StepCtl &c, const double E[4], double reltol, bool forced)
 {
-    const bool done = controller_decide(c, E, reltol, forced);
-    if (c.accepted) c.dtnext = controller_next(c.h, E, reltol);
+    const bool done = controller_decide<true>(c, E, reltol, forced);
+    if (c.accepted) c.dtnext = controller_next<true>(c.h, E, reltol);
     return done;
 }
 
