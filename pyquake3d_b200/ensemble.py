@@ -93,6 +93,20 @@ def ensemble_tasks(row0, task_rows):
     return task_row, task_fault, fault_task
 
 
+def ensemble_task_rows(row0, ctas, most):
+    """Rows per task on `ctas` co-resident CTAs: as few (in 16s, at most `most`) as give half the
+    CTAs a task, so that a small ensemble's row sums and element work spread over all SMs; more
+    while uneven faults make more tasks than CTAs, so that each task has one of its own; `most`,
+    in lock step, where that is not to be had.  us per step, B200: six faults of 12.6k rows 19.0
+    with 96 rows, 22.2 with 256, 44 in lock step with 32; 100 faults of
+    200 rows and 100 of 50 42 with 208, 141 in lock step with 176."""
+    sizes = np.diff(np.asarray(row0, dtype=np.int64))
+    rows = min(most, 16 * -(-int(sizes.sum()) // (16 * max(1, ctas // 2))))
+    while rows < most and int((-(-sizes // rows)).sum()) > ctas:
+        rows += 16
+    return min(rows, most)
+
+
 class Ensemble:
     """Independent faults (QDsim objects, host-initialized) stepped together."""
 
@@ -150,12 +164,7 @@ class Ensemble:
                        shear_loading=lambda s: s.shear_loading, normal_loading=lambda s: s.normal_loading,
                        vplc=lambda s: s.slipvC, cr0=lambda s: np.cos(s.rake0), sr0=lambda s: np.sin(s.rake0))
         self.t = {k: torch.tensor(np.ascontiguousarray(cat(g)), **f64) for k, g in getters.items()}
-        # tasks as short as gives half the co-resident grid a task (in 16s), so that a small
-        # ensemble's row sums and element work spread over all SMs, and all tasks get a CTA of
-        # their own (12.6k elements: 19.0 us per step kernel with 96 rows, 22.2 with 256; 44 in
-        # lock step with 32, more tasks than CTAs)
-        cap = max(1, self.L.pq3d_ens_grid(1 << 30) // 2)
-        rows = min(self.L.pq3d_ens_task_rows(), 16 * -(-n // (16 * cap)))
+        rows = ensemble_task_rows(self.struct.row0, self.L.pq3d_ens_grid(1 << 30), self.L.pq3d_ens_task_rows())
         task_row, task_fault, fault_task = ensemble_tasks(self.struct.row0, rows)
         self.n_tasks = T = len(task_fault)
         self.task_row = torch.tensor(task_row, device=dev)
