@@ -310,7 +310,7 @@ static int stress_host(const double *X, const double *Y, const double *Z, size_t
         return PQ3D_ERR_CUDA;
     }
     int rc = pq3d_stress_points(d, d + npt, d + 2 * npt, (int64_t)npt, d + 3 * npt, (int64_t)nsrc, Ss, Ds, Ts, mu,
-                                lam, hs ? 2 : 0, dS, dS + 6 * np, st);
+                                lam, hs ? 2 : 0, dS, strain ? dS + 6 * np : nullptr, st);
     if (rc != PQ3D_OK) return rc;
     const size_t bs = 6 * np * sizeof(double);
     if (packed) {
