@@ -238,11 +238,12 @@ static void fill_nan(double *a, size_t n)
 // one stream.  The reference calls its entry points for every row and column of
 // small blocks, so per-call allocations and copies would cost more than the work:
 // calls of up to 1 MB pack their inputs into the pinned buffer, which the kernel
-// reads and writes in place.  Per call against one copy each way (B200, full /
-// half space): 64 receivers 31 -> 21 / 67 -> 37 us, 1,000 37 -> 29 / 76 -> 47, 8,000
-// 89 -> 77 / 137 -> 104; larger calls are bound by the host's copies into the caller's
-// arrays either way.  Calls on a device are serialised by a mutex (the buffers are
-// shared).
+// reads and writes in place.  us per call, B200, one copy each way -> in place, on two
+// hosts: one source in the full space, 64 receivers 46 -> 36 and 45 -> 34, 1,000 52 -> 45 and
+// 50 -> 41, 6,000 89 -> 92 and 86 -> 76, 8,700 114 -> 117 and 107 -> 98; in the half space 56 -> 51 and
+// 141 -> 135 for 64 and 8,700 (first host); 64 sources 40 -> 31, 6,000 131 -> 131.  Larger calls are
+// bound by the host's copies into the caller's arrays either way.  Calls on a device are
+// serialised by a mutex (the buffers are shared).
 namespace {
 constexpr int kDropinDevices = 64;
 struct DropinStage {
