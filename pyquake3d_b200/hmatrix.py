@@ -199,6 +199,8 @@ def aca_start_indices(blocks, seed):
     pass, then again for the dip pass, src/Hmatrix.py:660-661 and :888-889), with
     a seeded legacy RandomState and blocks taken in list order."""
     sizes = [(len(b.row.indices), len(b.col.indices)) * 2 for b in blocks if b.aca]
+    if not sizes:
+        return []
     # one draw over the array of bounds gives the numbers of a draw per bound
     r = np.random.RandomState(seed).randint(np.array(sizes, dtype=np.int64).reshape(-1)) - 3
     return [((a, b), (c, d)) for a, b, c, d in r.reshape(-1, 4).tolist()]
@@ -301,6 +303,23 @@ def build_plan_arrays(struct, dense_recs, kS, kD, code, dense_chunk=64, v_chunk=
     lr_entries = int((3 * (ks + kd) * ((hi - lo) + nn)).sum())
     on = np.nonzero(ks + kd > 0)[0]                     # blocks with terms
     m, nn, row0, c0, lo, hi, ks, kd = (a[on] for a in (m, nn, row0, c0, lo, hi, ks, kd))
+    lr = dict(vitems=_fields(_lib.V_ITEM, 0), utasks=_fields(_lib.U_TASK, 0), n_vitems=0, n_utasks=0, n_slots=slot0,
+              n_tpart=0, kmax=0, u_size=0, v_size=0, pack=np.zeros(0, dtype=_PACK))
+    if len(on):
+        lr, rows = _lowrank_items(m, nn, row0, c0, lo, hi, ks, kd, on, cwl, v_chunk, u_rows, slot0)
+        slot_rows = np.concatenate([slot_rows, rows])
+    L = _leaf_lists(struct, slot_rows)
+    esz_d = 8 if code == 0 else 4
+    esz_l = {0: 8, 1: 4, 2: 2}[code]
+    dense_entries = int(np.sum(dense_recs["m"].astype(np.int64) * dense_recs["n"])) if len(dense_recs) else 0
+    nd = len(ditems)
+    return dict(ditems=_fields(_lib.DENSE_ITEM, 0) if nd == 0 else ditems, n_ditems=nd,
+                alg_bytes=dense_entries * 6 * esz_d + lr_entries * esz_l + 2 * n * esz_d + 3 * n * 8, **lr, **L)
+
+
+def _lowrank_items(m, nn, row0, c0, lo, hi, ks, kd, on, cwl, v_chunk, u_rows, slot0):
+    """The low-rank part of build_plan_arrays for the blocks with terms (their geometry, terms per
+    pass and numbers `on`), slots from slot0: (plan entries, slot owners)."""
     K, Q, lead = _cdiv(ks + kd, cwl) * cwl, 3 * (ks + kd), c0 % cwl
     ngv = _cdiv(nn + lead, cwl)
     nch = _cdiv(ngv, v_chunk)
@@ -326,21 +345,12 @@ def build_plan_arrays(struct, dense_recs, kS, kD, code, dense_chunk=64, v_chunk=
     nu = len(b)
     utasks = _fields(_lib.U_TASK, nu, off=u_off[b], m=m[b], r0=r0, r1=np.minimum(hi[b], r0 + u_rows), K=K[b], kS=ks[b],
                      kD=kd[b], Q=Q[b], tp=tp[b], nch=nch[b], slot=(slot - lo)[b])
-    slot_rows = np.concatenate([slot_rows, np.stack([slot, row0 + lo, hi - lo], axis=1)])
     pack = np.zeros(2 * len(on), dtype=_PACK)
     for k, v in dict(bi=on, u_off=u_off, v_off=v_off, K=K, Q=Q, kS=ks, kD=kd).items():
         pack[k] = np.repeat(v, 2)
     pack["pass_"] = np.tile([0, 1], len(on))
-    L = _leaf_lists(struct, slot_rows)
-    esz_d = 8 if code == 0 else 4
-    esz_l = {0: 8, 1: 4, 2: 2}[code]
-    dense_entries = int(np.sum(dense_recs["m"].astype(np.int64) * dense_recs["n"])) if len(dense_recs) else 0
-    nd = len(ditems)
-    return dict(ditems=_fields(_lib.DENSE_ITEM, 0) if nd == 0 else ditems, vitems=vitems, utasks=utasks,
-                n_ditems=nd, n_vitems=nv, n_utasks=nu, n_slots=n_slots, n_tpart=n_tpart,
-                kmax=int(K.max()) if len(K) else 0,
-                u_size=u_size, v_size=v_size, pack=pack, alg_bytes=dense_entries * 6 * esz_d + lr_entries * esz_l +
-                2 * n * esz_d + 3 * n * 8, **L)
+    return dict(vitems=vitems, utasks=utasks, n_vitems=nv, n_utasks=nu, n_slots=n_slots, n_tpart=n_tpart,
+                kmax=int(K.max()), u_size=u_size, v_size=v_size, pack=pack), np.stack([slot, row0 + lo, hi - lo], axis=1)
 
 
 def _dense_items(dense_recs, cwd, dense_off, dense_chunk):
@@ -478,6 +488,26 @@ def build_plan_arrays_mixed(struct, dense_recs, cls_lists, dense_chunk=16, v_chu
     ditems, slot_rows, slot0 = _dense_items(dense_recs, 4, dense_recs["off32"], dense_chunk)
     if counts is None:
         counts = np.array([[np.bincount(c, minlength=3) for c in cl] for cl in cls_lists], np.int64).reshape(-1, 2, 3)
+    lr = dict(vitems=_fields(_lib.V_ITEM_M, 0), vwarp=np.zeros(9, np.int32), vrows=_fields(_lib.V_ROW, 0),
+              utasks=_fields(_lib.U_TASK_M, 0), n_utasks=0, n_slots=slot0, n_tpart=0, n_scales=0, kmax=0,
+              u_sizes=[0, 0, 0], v_sizes=[0, 0, 0], pack=np.zeros(0, dtype=_PACK_M),
+              class_terms=np.zeros((3, 2), np.int64))
+    lr_bytes = 0
+    if counts.any():
+        lr, rows, lr_bytes = _lowrank_items_mixed(struct, counts, v_chunk, u_rows, slot0, nwarps or VMIX_WARPS)
+        slot_rows = np.concatenate([slot_rows, rows])
+    A = _leaf_lists(struct, slot_rows)
+    dense_entries = int(np.sum(dense_recs["m"].astype(np.int64) * dense_recs["n"])) if len(dense_recs) else 0
+    n = struct.n
+    nd = len(ditems)
+    A.update(ditems=_fields(_lib.DENSE_ITEM, 0) if nd == 0 else ditems, n_ditems=nd, n_vitems=int(lr["vwarp"][-1]),
+             stream=False, alg_bytes=dense_entries * 6 * 4 + lr_bytes + 2 * n * 4 + 3 * n * 8, **lr)
+    return A
+
+
+def _lowrank_items_mixed(struct, counts, v_chunk, u_rows, slot0, nwarps):
+    """The low-rank part of build_plan_arrays_mixed, slots from slot0: (plan entries, slot owners,
+    bytes of the factors)."""
     CW = np.array(MIXED_CW)
     m, nn, row0, c0, lo, hi = _block_geometry([b for b in struct.blocks if b.aca])
     on = np.nonzero(counts.sum(axis=(1, 2)) > 0)[0]              # blocks with terms
@@ -507,28 +537,21 @@ def build_plan_arrays_mixed(struct, dense_recs, cls_lists, dense_chunk=16, v_chu
     # one entry per (block, class) with rows, for the merged V items
     b, c = np.nonzero(K > 0)
     vitems, vwarp, vrows = _merged_v_items(c0[b], nn[b], c, v_off[b, c], Q[b, c], 3 * ks[b, c], tp[b, c], v_chunk,
-                                           nwarps or VMIX_WARPS)
+                                           nwarps)
     o, i = _expand(_cdiv(hi - lo, u_rows))
     r0 = lo[o] + i * u_rows
     nu = len(o)
     utasks = _fields(_lib.U_TASK_M, nu, off=u_off[o], m=m[o], r0=r0, r1=np.minimum(hi[o], r0 + u_rows),
                      slot=(slot - lo)[o], K=K[o], kS=ks[o], kD=kd[o], Q=Q[o], tp=tp[o], nch=nch[o], sb=sb[o])
-    slot_rows = np.concatenate([slot_rows, np.stack([slot, row0 + lo, hi - lo], axis=1)])
     pack = np.zeros(2 * len(on), dtype=_PACK_M)
     for k, v in dict(bi=on, u_off=u_off, v_off=v_off, kS=ks, kD=kd, Q=Q, K=K, sb=sb).items():
         pack[k] = np.repeat(v, 2, axis=0)
     pack["pass_"] = np.tile([0, 1], len(on))
-    A = _leaf_lists(struct, slot_rows)
-    dense_entries = int(np.sum(dense_recs["m"].astype(np.int64) * dense_recs["n"])) if len(dense_recs) else 0
-    n = struct.n
     lr_bytes = int((Q * ((hi - lo) + nn)[:, None] * np.array(MIXED_BYTES)).sum() + 4 * scaled.sum())
-    nd = len(ditems)
-    A.update(ditems=_fields(_lib.DENSE_ITEM, 0) if nd == 0 else ditems, vitems=vitems, vrows=vrows, vwarp=vwarp,
-             utasks=utasks, n_ditems=nd, n_vitems=int(vwarp[-1]), n_utasks=nu, n_slots=n_slots, n_tpart=n_tpart,
-             n_scales=n_scales, kmax=int(K.sum(axis=1).max()) if len(K) else 0, u_sizes=u_size, v_sizes=v_size,
-             pack=pack, stream=False, class_terms=np.stack([ks.sum(axis=0), kd.sum(axis=0)], axis=1),
-             alg_bytes=dense_entries * 6 * 4 + lr_bytes + 2 * n * 4 + 3 * n * 8)
-    return A
+    return dict(vitems=vitems, vrows=vrows, vwarp=vwarp, utasks=utasks, n_utasks=nu, n_slots=n_slots, n_tpart=n_tpart,
+                n_scales=n_scales, kmax=int(K.sum(axis=1).max()), u_sizes=u_size, v_sizes=v_size, pack=pack,
+                class_terms=np.stack([ks.sum(axis=0), kd.sum(axis=0)], axis=1)), \
+        np.stack([slot, row0 + lo, hi - lo], axis=1), lr_bytes
 
 
 VMIX_WARPS = 8 * 148 * 4      # k_v_mixed warps when no device says otherwise (B200, 4 CTAs per SM)
@@ -870,6 +893,10 @@ class DeviceHMatrix:
     def _run_aca(self):
         """Batched ACA over all admissible blocks; ranks and FP64 factors kept per task."""
         torch = self.torch
+        if not self.aca_blocks:
+            self.aca_ranks, self.aca_flags = np.zeros(0, np.int32), np.zeros(0, np.int32)
+            self.aca_ws, self.task_ws = [], workspace_table(0)
+            return
         starts = getattr(self.s, "aca_starts", None)
         if starts is None:
             starts = aca_start_indices(self.s.blocks, self.aca_seed)
@@ -877,9 +904,9 @@ class DeviceHMatrix:
         nt = 2 * len(blocks)                     # tasks: strike and dip pass of every block
         m, n = (np.repeat(v, 2) for v in _block_geometry(blocks)[:2])
         start = np.array(starts, dtype=np.int64).reshape(-1, 2)
-        none = [np.zeros(1, np.int32)]           # row and column lists stored separately
-        self.rowlist = torch.from_numpy(np.concatenate([b.row.indices for b in blocks] or none).astype(np.int32)).to(self.dev)
-        self.collist = torch.from_numpy(np.concatenate([b.col.indices for b in blocks] or none).astype(np.int32)).to(self.dev)
+        # row and column lists stored separately
+        self.rowlist = torch.from_numpy(np.concatenate([b.row.indices for b in blocks]).astype(np.int32)).to(self.dev)
+        self.collist = torch.from_numpy(np.concatenate([b.col.indices for b in blocks]).astype(np.int32)).to(self.dev)
         ro, co = self._row_offsets()
         self.aca_ranks = np.zeros(nt, dtype=np.int32)
         self.aca_flags = np.zeros(nt, dtype=np.int32)
@@ -954,6 +981,8 @@ class DeviceHMatrix:
         Vbuf = torch.zeros(max(A["v_size"], 8), dtype=lr_dtype, device=self.dev)
         # pack every ACA task into the layout, one launch per workspace batch
         K = A["pack"]
+        if len(K) == 0:
+            return self._finish_plan(dtype, A, Ubuf, Vbuf)
         ti = 2 * K["bi"] + K["pass_"]
         rec = self._task_records(_lib.PACK_TASK, ti)
         for k in ("u_off", "v_off", "kS", "kD", "K", "Q"):
@@ -1025,6 +1054,40 @@ class DeviceHMatrix:
         torch = self.torch
         if self.dense32 is None:
             raise _lib.Pq3dError("the mixed plan needs the FP32 dense blocks: request it in assemble(want=...)")
+        L = self.L
+        st = self._stream
+        offs, tmap = np.zeros(1, np.int64), np.zeros(1, np.int32)
+        if self.aca_blocks:
+            rec, offs, tmap = self._term_classes()
+        self.mixed_tmap = tmap[:int(offs[-1])]
+        A = self._mixed_arrays(self.mixed_tmap & 3, offs)
+        # INT8-class entries are stored as b + 128: the fill 128 decodes to zero, so padding
+        # columns (a block's lead and tail columns, its K padding) contribute nothing
+        tdt, fill = (torch.float32, torch.float16, torch.uint8), (0, 0, 128)
+        Ub = [torch.full((max(int(A["u_sizes"][c]), 16),), fill[c], dtype=tdt[c], device=self.dev) for c in range(3)]
+        Vb = [torch.full((max(int(A["v_sizes"][c]), 16),), fill[c], dtype=tdt[c], device=self.dev) for c in range(3)]
+        scales = torch.zeros(max(A["n_scales"], 4), dtype=torch.float32, device=self.dev)
+        d_tmap = torch.from_numpy(tmap).to(self.dev)
+        K = A["pack"]                              # blocks with terms
+        if len(K):
+            if A.get("stream"):
+                K = np.array([tuple(k) for k in K], dtype=_PACK_M)
+            ti = 2 * K["bi"] + K["pass_"]
+            rec = rec[ti]
+            for k in ("u_off", "v_off", "kS", "kD", "Q", "K", "sb"):
+                rec[k] = K[k]
+            for wi, d_rec, k in self._by_workspace(rec, ti):
+                check(L.pq3d_aca_pack_mixed(ptr(d_rec), k, ptr(self.aca_ws[wi]), ptr(self.rowlist), ptr(self.collist),
+                                            ptr(self.iperm), ptr(d_tmap), ptr(Ub[0]), ptr(Ub[1]), ptr(Ub[2]), ptr(Vb[0]),
+                                            ptr(Vb[1]), ptr(Vb[2]), ptr(scales), st), "pq3d_aca_pack_mixed")
+        A["mixed"] = dict(U=Ub, V=Vb, scales=scales, tol=self.mixed_tol, class_terms=A["class_terms"].tolist())
+        return self._finish_plan("mixed", A, Ub[0], Vb[0])
+
+    def _term_classes(self):
+        """Packing records of all tasks, the tasks' term offsets, and every term's class and
+        position among its task's terms of that class (class | position << 2), from the terms'
+        weights."""
+        torch = self.torch
         n = self.n
         L = self.L
         st = self._stream
@@ -1053,28 +1116,7 @@ class DeviceHMatrix:
         pos[order] = _expand(np.bincount(key, minlength=3 * len(tasks)))[1]
         tmap = np.zeros(max(len(cls), 1), np.int32)
         tmap[:len(cls)] = cls | (pos << 2)
-        self.mixed_tmap = tmap[:len(cls)]
-        A = self._mixed_arrays(cls, offs)
-        # INT8-class entries are stored as b + 128: the fill 128 decodes to zero, so padding
-        # columns (a block's lead and tail columns, its K padding) contribute nothing
-        tdt, fill = (torch.float32, torch.float16, torch.uint8), (0, 0, 128)
-        Ub = [torch.full((max(int(A["u_sizes"][c]), 16),), fill[c], dtype=tdt[c], device=self.dev) for c in range(3)]
-        Vb = [torch.full((max(int(A["v_sizes"][c]), 16),), fill[c], dtype=tdt[c], device=self.dev) for c in range(3)]
-        scales = torch.zeros(max(A["n_scales"], 4), dtype=torch.float32, device=self.dev)
-        d_tmap = torch.from_numpy(tmap).to(self.dev)
-        K = A["pack"]                              # blocks with terms
-        if self.mixed_stream and A.get("stream"):
-            K = np.array([tuple(k) for k in K], dtype=_PACK_M)
-        ti = 2 * K["bi"] + K["pass_"]
-        rec = rec[ti]
-        for k in ("u_off", "v_off", "kS", "kD", "Q", "K", "sb"):
-            rec[k] = K[k]
-        for wi, d_rec, k in self._by_workspace(rec, ti):
-            check(L.pq3d_aca_pack_mixed(ptr(d_rec), k, ptr(self.aca_ws[wi]), ptr(self.rowlist), ptr(self.collist),
-                                        ptr(self.iperm), ptr(d_tmap), ptr(Ub[0]), ptr(Ub[1]), ptr(Ub[2]), ptr(Vb[0]),
-                                        ptr(Vb[1]), ptr(Vb[2]), ptr(scales), st), "pq3d_aca_pack_mixed")
-        A["mixed"] = dict(U=Ub, V=Vb, scales=scales, tol=self.mixed_tol, class_terms=A["class_terms"].tolist())
-        return self._finish_plan("mixed", A, Ub[0], Vb[0])
+        return rec, offs, tmap
 
     def _mixed_arrays(self, cls, offs):
         """Plan arrays from every term's class (task order) and the tasks' term offsets."""
