@@ -163,14 +163,15 @@ __global__ void __launch_bounds__(MT) k_mlp_fwd(const float *__restrict__ P, con
     }
 }
 
-// part[blockIdx.x][NPP]: this CTA's share of every gradient (and of the loss) over its tiles.
+// part[blockIdx.x][NPP]: this CTA's share of every gradient over its tiles; loss_part, with the
+// same stride, its share of the loss.
 // The W2 gradient (64 x 64, a sum over the tile's samples) is 4 x 4 per thread, units
 // threadIdx / 16 + 16 a and inputs threadIdx % 16 + 16 b, so the 16-byte reads along the
 // samples fall in different banks; the other gradients stay with the thread that holds the
 // unit and are summed over its 16 lanes at the end.
 __global__ void __launch_bounds__(MT, 2) k_mlp_grad(const float *__restrict__ P, const float *__restrict__ X, int xstride,
                                                     const float *__restrict__ T, int tstride, int B,
-                                                    float *__restrict__ part)
+                                                    float *__restrict__ part, float *__restrict__ loss_part)
 {
     __shared__ __align__(16) Weights w;
     __shared__ __align__(16) float h1[H * SST];
@@ -283,7 +284,7 @@ __global__ void __launch_bounds__(MT, 2) k_mlp_grad(const float *__restrict__ P,
         gl += __shfl_xor_sync(0xffffffffu, gl, 16);
         if (lane == 0) {
             o[OFF_B3] = gb3;
-            o[NP] = gl;
+            loss_part[(int64_t)blockIdx.x * NPP] = gl;
         }
     }
 }
@@ -295,8 +296,10 @@ struct Adam {
 };
 
 // G[p] = sum of the CTAs' shares: 32 parameters per CTA, eight threads a parameter, each
-// over every eighth share in order, so all loads are in flight at once; then Adam.
-__global__ void __launch_bounds__(256) k_mlp_reduce(const float *__restrict__ part, int nblk, float *__restrict__ G,
+// over every eighth share in order, so all loads are in flight at once; then Adam.  A single
+// share may stand in G itself, so the shares are not read through the read-only path; past L1 (they
+// come from other SMs) they take no longer by it (296 shares: 6 us, 8 through L1).
+__global__ void __launch_bounds__(256) k_mlp_reduce(const float *part, const float *loss_part, int nblk, float *G,
                                                     float *__restrict__ loss, Adam A)
 {
     __shared__ float red[8][33];
@@ -304,8 +307,9 @@ __global__ void __launch_bounds__(256) k_mlp_reduce(const float *__restrict__ pa
     const int p = blockIdx.x * 32 + c;
     float s = 0.0f;
     if (p <= NP) {
+        const float *q = p < NP ? part + p : loss_part;
 #pragma unroll 8
-        for (int k = r; k < nblk; k += 8) s += part[(int64_t)k * NPP + p];
+        for (int k = r; k < nblk; k += 8) s += __ldcg(q + (int64_t)k * NPP);
     }
     red[r][c] = s;
     __syncthreads();
@@ -328,34 +332,35 @@ __global__ void __launch_bounds__(256) k_mlp_reduce(const float *__restrict__ pa
     A.P[p] -= A.lr * mh / (sqrtf(vh) + A.eps);
 }
 
-int64_t scratch_floats(int B)
-{
-    const int64_t f = (int64_t)4 * H * B + 2 * (int64_t)B;
-    return f > NPP ? f : NPP;
-}
+// 258 floats a sample, which callers have always allocated: shares for one CTA per tile from 36
+// samples on.
+int64_t scratch_floats(int B) { return (int64_t)4 * H * B + 2 * (int64_t)B; }
 
-// CTAs of a gradient over B samples: one per tile, as many as the scratch holds shares for.
+// CTAs of a gradient over B samples: one per tile, as many as the scratch holds shares for.  One
+// CTA needs no scratch but for the loss: its share is the gradient.
 int grad_ctas(int B)
 {
     int64_t n = ((int64_t)B + TS - 1) / TS;
     const int64_t fit = scratch_floats(B) / NPP;
     n = n < fit ? n : fit;
-    return (int)(n < MAX_CTAS ? n : MAX_CTAS);
+    n = n < MAX_CTAS ? n : MAX_CTAS;
+    return (int)(n > 1 ? n : 1);
 }
 
 int gradient(const float *P, const float *X, int xstride, const float *T, int tstride, int B, float *scratch, float *G,
              float *loss, const Adam &A, cudaStream_t stream)
 {
     const int n = grad_ctas(B);
-    k_mlp_grad<<<n, MT, 0, stream>>>(P, X, xstride, T, tstride, B, scratch);
-    k_mlp_reduce<<<(NP + 32) / 32, 256, 0, stream>>>(scratch, n, G, loss, A);
+    float *part = n > 1 ? scratch : G, *loss_part = n > 1 ? scratch + NP : scratch;
+    k_mlp_grad<<<n, MT, 0, stream>>>(P, X, xstride, T, tstride, B, part, loss_part);
+    k_mlp_reduce<<<(NP + 32) / 32, 256, 0, stream>>>(part, loss_part, n, G, loss, A);
     return pq3d_launch_status();
 }
 }  // namespace
 
 PQ3D_EXPORT int pq3d_mlp_param_count(void) { return NP; }
 
-// Scratch for a batch of B samples (the CTAs' shares of the gradient).
+// Scratch for a batch of B samples.
 PQ3D_EXPORT int64_t pq3d_mlp_scratch_floats(int B) { return scratch_floats(B); }
 
 // y = MLP(X) for B samples (X rows of xstride floats, the first 5 used).
