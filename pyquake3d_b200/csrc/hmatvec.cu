@@ -1110,8 +1110,8 @@ __global__ void __launch_bounds__(128) k_t_gather(const TGather *__restrict__ gs
 
 // ------------------------------------------------------------------ kernel 3
 // y[3i+c] = sum of row i's slots + add[c][i] (FP64): R rows per CTA (rowsum.cuh).  1,936 rows
-// of 121 FP64 slots 48.7 -> 6.3 us, 9,000 of 40 FP32 slots 9.8 -> 5.3, 60k of 56 FP32 slots
-// 22.0 -> 15.8 us against one thread a row with four entries in flight.
+// of 121 FP64 slots 48.7 -> 5.4 us, 9,000 of 40 FP32 slots 9.8 -> 4.8, 60k of 56 FP32 slots
+// 22.0 -> 15.4 us against one thread a row with four entries in flight.
 template <typename TA>
 __global__ void __launch_bounds__(256)
 k_rowsum(int n, int R, const int32_t *__restrict__ leaf_of_row, const int32_t *__restrict__ leaf_ptr,
@@ -1131,8 +1131,8 @@ k_rowsum(int n, int R, const int32_t *__restrict__ leaf_of_row, const int32_t *_
 }
 
 // 16 rows per CTA until that gives two CTAs per SM, then 64: us for 16 / 32 / 64 / 128 rows at
-// 1,936 rows FP64 6.3 / 8.9 / 14.7 / 47, at 9,000 FP64 - / 6.0 / 6.1 / 7.6,
-// at 60k FP32 - / 17.6 / 15.8 / 16.1.
+// 1,936 rows FP64 5.4 / 6.3 / 9.0 / 17.4, at 9,000 FP64 8.9 / 6.3 / 5.7 / 5.4 and FP32 6.7 / 5.0 / 4.8 / 5.5,
+// at 60k FP32 30.7 / 19.2 / 15.5 / 14.4.
 template <typename TA>
 static void launch_rowsum(const int n, const int32_t *leaf_of_row, const int32_t *leaf_ptr, const int32_t *leaf_off,
                           const TA *slots, const double *add0, const double *add1, const double *add2, double *y,

@@ -42,19 +42,13 @@ struct RkArgs {
     double h_in;         // > 0: the step's trial size (instead of ctrl[0])
 };
 
-#ifndef PQ3D_RK_THREADS
-#define PQ3D_RK_THREADS 256
-#endif
 // Two 256-thread CTAs per SM, R rows per CTA (rs_rows): at 60k elements one element per thread,
 // below that as few rows per CTA as fill the grid, so that all SMs share the latency-bound
 // element work and every thread the row sums.  B200, us per launch, against 256 rows per CTA and
-// unrolled stages: 1,936 elements 43.5 -> 19.0, 5,000 22.5 -> 17.7, 20,480 24.0 -> 22.5, 60k 42.9 -> 35.6.
+// unrolled stages: 1,936 elements 44.0 -> 18.8, 5,120 22.5 -> 17.7, 20,480 24.3 -> 22.3, 60k 43.7 -> 34.5.
 // Cycles of a launch at 20,480 (clock64 stamps): row sums 9,600, stages 14,200 (seven derivatives
 // of 930, their combinations 430 each), grid maximum 6,300, accept 5,400, end of step 3,000.
-#ifndef PQ3D_RK_MINB
-#define PQ3D_RK_MINB 2
-#endif
-constexpr int RK_THREADS = PQ3D_RK_THREADS;   // CTA size of the step kernel
+constexpr int RK_THREADS = 256;   // CTA size of the step kernel (fault_max4 reduces eight warps)
 
 struct WholeGrid {
     const RkArgs &A;
@@ -69,7 +63,7 @@ struct WholeGrid {
 
 // TA: type of the matvec's slots (a kernel each, for half the code).
 template <typename TA>
-__global__ void __launch_bounds__(RK_THREADS, PQ3D_RK_MINB) k_rk_step(RkArgs A)
+__global__ void __launch_bounds__(RK_THREADS, 2) k_rk_step(RkArgs A)
 {
     const int n = A.n;
     // R rows per CTA, one per thread; the other threads take part in the row sums

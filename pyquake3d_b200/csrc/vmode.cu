@@ -35,7 +35,7 @@ struct VArgs {
     double *V;            // 2 x n: latest slip rates (previous-rate seed)
     void *x;              // deficit of the next matvec (device layout of hm_layout.cuh)
     double *ctrl;         // control block (pq3d.h)
-    double *blk;          // 2 * grid scratch
+    double *blk;          // pq3d_vmode_grid(n) doubles scratch
     unsigned *bar;        // bar[0]: stage-7 completion count (zeroed once)
     unsigned long long *stats;  // [0] Newton iterations, [1] solves, [2] max iterations, [3] fallbacks
     const float *mlp;     // MLP parameters (4609 floats) or null
@@ -215,9 +215,10 @@ __device__ inline void write_x(const VArgs &A, int64_t i, double d1, double d2)
 }
 
 // Two lanes an element, one traction component each: the stage is a chain of some ten FP64
-// transcendentals per component, and with both in one thread (and a copy of the solve for each)
-// it took 11.5 us for 9,000 elements on 71 CTAs, @@ now.  The Newton counters go up once per
-// CTA; one atomic per warp and counter queued on the same words.
+// transcendentals per component.  Launched behind the row reduction's start it waits for its end:
+// the two take 11.2 us for 9,000 elements, 6.3 of them after the reduction, against 21.0 and 12.0
+// with a plain launch and both components in one thread (and a copy of the solve for each).  The
+// Newton counters go up once per CTA; one atomic per warp and counter queued on the same words.
 __global__ void __launch_bounds__(VM_THREADS) k_vmode_stage(VArgs A, int s)
 {
     __shared__ double red[VM_THREADS / 32][2];

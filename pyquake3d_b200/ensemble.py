@@ -3,7 +3,8 @@
 The reference simulates one fault per (MPI) job; a batch of independent faults
 is run as separate jobs.  Here a batch shares the device: the H-matrices of all
 faults form one block-diagonal operator (one set of matvec work items, one
-launch), and one cooperative step kernel (pq3d_ens_step) advances every fault
+launch), and one cooperative step kernel (pq3d_ens_step_faults, or pq3d_ens_step
+where there are more CTA tasks than co-resident CTAs) advances every fault
 with its own DP5(4) step-size controller, exactly as QDsim.simu_forward
 (src/QDsim.py:892-996) advances a single fault.
 
@@ -98,8 +99,8 @@ def ensemble_task_rows(row0, ctas, most):
     CTAs a task, so that a small ensemble's row sums and element work spread over all SMs; more
     while uneven faults make more tasks than CTAs, so that each task has one of its own; `most`,
     in lock step, where that is not to be had.  us per step, B200: six faults of 12.6k rows 19.0
-    with 96 rows, 22.2 with 256, 44 in lock step with 32; 100 faults of
-    200 rows and 100 of 50 42 with 208, 141 in lock step with 176."""
+    with 96 rows, 22.2 with 256, 44 in lock step with 32; 100 faults of 200 rows and 100 of 50
+    42 with 208, 141 in lock step with 176."""
     sizes = np.diff(np.asarray(row0, dtype=np.int64))
     rows = min(most, 16 * -(-int(sizes.sum()) // (16 * max(1, ctas // 2))))
     while rows < most and int((-(-sizes // rows)).sum()) > ctas:

@@ -404,7 +404,8 @@ MIXED_EPS = (2.0 ** -24, 2.0 ** -11, 0.5 / 127.0)
 
 
 def classify_terms(wS, wD, tol):
-    """Classes (0 FP32, 1 FP16, 2 INT8) of one block's ACA terms from their weights
+    """The rule of classify_blocks, stated for one block (the plans use the former; tests
+    compare the two): classes (0 FP32, 1 FP16, 2 INT8) of the block's ACA terms from their weights
     w = max_i(|u_i| / R_i) ||v||_1 (strike terms wS, dip terms wD, in ACA order).
 
     A term needs FP32 when 2 eps_FP16 w > tol (quantising u and v to FP16 would move a
@@ -474,8 +475,8 @@ def build_plan_arrays_mixed(struct, dense_recs, cls_lists, dense_chunk=16, v_chu
     """Work items, slot layout and packing records of the mixed storage (code 3):
     FP32 dense items as in the FP32 plan; per low-rank block and term class c
     (FP32, FP16, INT8) the class's own U / V arrays with column groups MIXED_CW[c].
-    cls_lists[bi] = (cls_S, cls_D) from classify_terms, or counts[bi, pass, class] terms
-    of each class (class_counts).  Pure numpy.
+    counts[bi, pass, class]: terms of each class (class_counts of classify_blocks), or
+    cls_lists[bi] = (cls_S, cls_D), the classes of one block's terms.  Pure numpy.
 
     stream=True lays the work out for the persistent bulk-copy kernel k_stream:
     StreamTask lists of phase A (dense tasks of at most STREAM_DENSE_ROWS rows and
@@ -808,7 +809,7 @@ class DeviceHMatrix:
         """halfspace: 0 full space; 1 half space, a triangle side along z adds no
         free-surface term; 2 half space with the side handling of the reference's
         compiled library (the values its H-matrix assembly uses).  mixed_tol: the
-        term-class tolerance of the "mixed" storage (classify_terms)."""
+        term-class tolerance of the "mixed" storage (classify_blocks)."""
         self.mixed_tol = float(mixed_tol)
         self.mixed_stream = False      # mixed storage: True selects the bulk-copy (streamed) kernels
         self.use_plan_cache = True
