@@ -283,16 +283,21 @@ __device__ __forceinline__ void smem_vec<double, 2>(const double *p, double *o)
 }
 
 // Start bringing a U task's rows into L2: one bulk prefetch per column group and component
-// (rows [r0, r1), 16 B each).  They do not depend on the V partials the task waits for.  Used by
-// the FP32 tasks (product of 20,480 elements 137.9 -> 133.8 us, 9,000 61.9 -> 60.9, 60k 706 either
-// way); BF16 (20,480: 104.6 -> 106.5) and FP64 ones (60k: 1,438 -> 1,589) lose by it, and so does
-// every type when only the first wave's tasks prefetch.
+// (rows [r0, r1), 16 B each), the first PREFETCH_BYTES of them.  They do not depend on the V
+// partials the task waits for.  Used by the FP32 tasks.  The limit: some 600 resident CTAs with
+// more than that (blocks of high rank) push one another's rows out of L2 again.  us without / with
+// all rows / with 96 KB, planar faults 8,820 elements 58.4 / 52.4 / 52.4, 20,480 128.2 / 122.0 / 122.0,
+// curved ones 9,108 82.5 / 74.1 / 75.4, 19,712 184 / 189 / 182, 60k 671 / 673 / 667 (64 KB: 77 and 178 at
+// 9,108 and 19,712, 128 KB: 75 and 185).  BF16 (20,480: 104.6 -> 106.5) and FP64 tasks (60k: 1,438 -> 1,589)
+// lose by it, and so does every type when only the first wave's tasks prefetch.
+constexpr int PREFETCH_BYTES = 96 * 1024;
+
 __device__ __forceinline__ void prefetch_u_rows(const void *U, int64_t off_bytes, int m, int r0, int r1, int ngroups,
                                                 int first, int stride)
 {
     const int nb = (r1 - r0) * 16;
     if (nb <= 0) return;
-    for (int e = first; e < 3 * ngroups; e += stride) {
+    for (int e = first; e < 3 * ngroups && (int64_t)e * nb < PREFETCH_BYTES; e += stride) {
         const unsigned char *p = (const unsigned char *)U + off_bytes + ((int64_t)e * m + r0) * 16;
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(nb) : "memory");
     }
