@@ -1135,18 +1135,6 @@ k_rowsum(int n, int R, const int32_t *__restrict__ leaf_of_row, const int32_t *_
     });
 }
 
-// 16 rows per CTA until that gives two CTAs per SM, then 64: us for 16 / 32 / 64 / 128 rows at
-// 1,936 rows FP64 5.4 / 6.3 / 9.0 / 17.4, at 9,000 FP64 8.9 / 6.3 / 5.7 / 5.4 and FP32 6.7 / 5.0 / 4.8 / 5.5,
-// at 60k FP32 30.7 / 19.2 / 15.5 / 14.4.
-template <typename TA>
-static void launch_rowsum(const int n, const int32_t *leaf_of_row, const int32_t *leaf_ptr, const int32_t *leaf_off,
-                          const TA *slots, const double *add0, const double *add1, const double *add2, double *y,
-                          cudaStream_t st)
-{
-    const int R = n <= 16 * 2 * 148 ? 16 : 64;
-    k_rowsum<TA><<<(n + R - 1) / R, 256, 0, st>>>(n, R, leaf_of_row, leaf_ptr, leaf_off, slots, add0, add1, add2, y);
-}
-
 // ------------------------------------------------------------------ host entry
 // Packed operator description (device pointers) -- mirrors the Python HM_PLAN record.
 struct HmPlan {
@@ -1193,6 +1181,21 @@ PQ3D_EXPORT size_t pq3d_item_bytes(int kind)
     case 10: return sizeof(VRowRec);
     }
     return 0;
+}
+
+// 16 rows per CTA until that gives two CTAs per SM, then 64: us for 16 / 32 / 64 / 128 rows at
+// 1,936 rows FP64 5.4 / 6.3 / 9.0 / 17.4, at 9,000 FP64 8.9 / 6.3 / 5.7 / 5.4 and FP32 6.7 / 5.0 / 4.8 / 5.5,
+// at 60k FP32 30.7 / 19.2 / 15.5 / 14.4.  Few rows with lists of a batch or less (a plan's n_slots / n
+// entries a row) take one thread each, with no sums to meet: 56 to 256 rows 2.8-3.1 -> 2.5-2.9 us (the
+// reduction with a thread a row throughout: 1.9-2.5, but 3.4 -> 5.3 at 256 FP64 rows of longer lists).
+template <typename TA>
+static void launch_rowsum(const HmPlan &P, const TA *slots, const double *add0, const double *add1, const double *add2,
+                          double *y, cudaStream_t st)
+{
+    const int n = P.n;
+    const bool few = n <= 256 && P.n_slots > 0 && P.n_slots <= (int64_t)pq3d::RS_BATCH * n;
+    const int R = few ? 256 : n <= 16 * 2 * 148 ? 16 : 64;
+    k_rowsum<TA><<<(n + R - 1) / R, 256, 0, st>>>(n, R, P.leaf_of_row, P.leaf_ptr, P.leaf_off, slots, add0, add1, add2, y);
 }
 
 template <typename TD, typename TL, typename TA>
@@ -1253,7 +1256,7 @@ static int run_matvec(const HmPlan &P, const TA *x, TA *slots, TA *tpart, const 
                                           (const TA *)tpart));
         }
     }
-    if (y) launch_rowsum<TA>(P.n, P.leaf_of_row, P.leaf_ptr, P.leaf_off, slots, add0, add1, add2, y, st);
+    if (y) launch_rowsum<TA>(P, slots, add0, add1, add2, y, st);
     return pq3d_launch_status();
 }
 
@@ -1292,7 +1295,7 @@ static int run_matvec_mixed(const HmPlan &P, const float *x, float *slots, float
                                       (const __half *)P.U16, (const uint8_t *)P.U8, x, slots, (const float *)tpart,
                                       P.scales));
     }
-    if (y) launch_rowsum<float>(P.n, P.leaf_of_row, P.leaf_ptr, P.leaf_off, slots, add0, add1, add2, y, st);
+    if (y) launch_rowsum<float>(P, slots, add0, add1, add2, y, st);
     return pq3d_launch_status();
 }
 
@@ -1331,7 +1334,7 @@ static int run_matvec_stream(const HmPlan &P, const float *x, float *slots, floa
         A.cta_ptr = P.cta_b;
         k_stream<<<(unsigned)P.ncta_b, ST_THREADS, sm, st>>>(A);
     }
-    if (y) launch_rowsum<float>(P.n, P.leaf_of_row, P.leaf_ptr, P.leaf_off, slots, add0, add1, add2, y, st);
+    if (y) launch_rowsum<float>(P, slots, add0, add1, add2, y, st);
     return pq3d_launch_status();
 }
 
