@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(256) k_mlp_reduce(const float *part, const flo
 #pragma unroll
     for (int k = 0; k < 8; ++k) s += red[k][c];
     if (p == NP) {
-        if (loss) *loss += s;
+        if (loss) atomicAdd(loss, s);      // batches of several streams may share the sum
         return;
     }
     G[p] = s;
